@@ -90,6 +90,8 @@ extern "C" int gbx_device_info(int *num_sms_out, int *arch)
 // float  rows (3a+c)*N + n : r_a[c]    (a = 12, 23, 31)
 //        rows (9 + 3s + c)*N + n, (18 + 3s + c)*N + n : P_s[c]/c as a float pair hi, lo
 //        rows (27 + 3a + c)*N + n : r_a[c] - (float)r_a[c] (the pair form's tails)
+// double rows (36 + c)*N + n, c = 0, 1 : P_1[c]/c rounded to a multiple of 2^-17 s, and
+//        rows (38 + c)*N + n : the rest (the FP64 form's exact products with k)
 __global__ void orbit_table_kernel(double *tab, const double *pos, int N, double L)
 {
     int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -105,6 +107,11 @@ __global__ void orbit_table_kernel(double *tab, const double *pos, int N, double
             tab[(size_t)(3 * s + c) * N + n] = pc;
             tf[(size_t)(9 + 3 * s + c) * N + n] = hi;
             tf[(size_t)(18 + 3 * s + c) * N + n] = (float)(pc - (double)hi);
+            if (s == 0 && c < 2) {
+                const double ph = rint(pc * 131072.0) / 131072.0;
+                tab[(size_t)(36 + c) * N + n] = ph;
+                tab[(size_t)(38 + c) * N + n] = pc - ph;
+            }
         }
     for (int c = 0; c < 3; c++) {
         // gbgpu.py:424-427: r12 = (P2 - P1)/L, r23 = (P3 - P2)/L, r31 = -(P3 - P1)/L
@@ -126,7 +133,7 @@ __global__ void orbit_table_kernel(double *tab, const double *pos, int N, double
 extern "C" size_t gbx_orbit_table_bytes(int N)
 {
     if (N <= 0) return 0;
-    return (size_t)N * (18 * sizeof(double) + 36 * sizeof(float));
+    return (size_t)N * (22 * sizeof(double) + 36 * sizeof(float));
 }
 
 extern "C" int gbx_orbit_table(void *table, const double *sc_pos, int N, double armlength,

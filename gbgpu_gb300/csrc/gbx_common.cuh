@@ -20,8 +20,10 @@ __host__ __device__ __forceinline__ int tile_pack(int tile, int lg, int minp)
     return p > kMaxPack ? kMaxPack : p;
 }
 constexpr int kTwN = 8192;         // twiddle table period (largest supported N)
+constexpr int kScN = 256;          // entries of the sin/cos tables (steps of pi/128)
 constexpr double kPi = 3.141592653589793238462643383279502884;
 constexpr double kTwoPi = 6.283185307179586476925286766559005768;
+constexpr double kTwoPiLo = 2.4492935982947064e-16;   // 2 pi - double(2 pi)
 constexpr double kInvTwoPi = 0.159154943091895335768883763372514362;
 constexpr double kCSI = 299792458.0;
 

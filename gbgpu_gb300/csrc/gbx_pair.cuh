@@ -159,8 +159,6 @@ __device__ __forceinline__ double pd(dfl a) { return (double)a.h + (double)a.l; 
 // (below 5e-15), combined by the angle-addition formulas.  pi/128 = C1 + C2
 // + C3 with C1 of 12 significant bits, so j C1 is exact for |j| < 4096 and
 // x.h - j C1 is formed exactly by TwoSum.
-constexpr int kScN = 256;
-
 __device__ __forceinline__ void sincos_pair(dfl x, const float4 *__restrict__ tab, dfl &c, dfl &s)
 {
     constexpr float kInv = 40.743663787841797f;     // 128/pi (picks j only)

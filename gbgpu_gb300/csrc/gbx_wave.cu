@@ -23,6 +23,7 @@ __device__ double2 g_tw_d[kTwN / 2];
 __device__ float2 g_tw_f[kTwN / 2];
 __device__ float4 g_tw_p[kTwN / 2];   // the same twiddles as float pairs (c.h, c.l, s.h, s.l)
 __device__ float4 g_sc_p[256];        // cos, sin of j pi/128 as float pairs (pair form)
+__device__ double2 g_sc_d[256];       // cos, sin of j pi/128 (FP64 form)
 
 __global__ void tw_init_kernel()
 {
@@ -40,6 +41,7 @@ __global__ void tw_init_kernel()
         sincospi((double)m / 128.0, &s, &c);
         const dfl cp = df_from(c), sp = df_from(s);
         g_sc_p[m] = make_float4(cp.h, cp.l, sp.h, sp.l);
+        g_sc_d[m] = make_double2(c, s);
     }
 }
 
@@ -57,7 +59,10 @@ struct __align__(16) Bin {
     double k[3];
     union {
         struct {
-            double ep[6], ec[6];   // e+ and ex, order xx yy zz xy xz yz (FP64 form)
+            double up[3], vp[3];   // u and v rotated by the polarisation angle (FP64 form)
+            double ap4, ci;        // (1 + cos^2 iota)/4, cos iota
+            double kh[2], kl[2];   // x and y of k: multiples of 2^-26, and the rest
+            double pf2, p3f3;      // 2 pi fdot, pi fddot
         } q;
         struct {
             dfl ud[3], vd[2];      // u and v (v has no z component) as pairs (pair form)
@@ -109,6 +114,8 @@ struct KParams {
     double fstar;                  // c / (2 pi L)
     dfl stepd[GBX_MAX_LOG2N + 1];  // T / 2^k as float pairs (exact: division by a power of two)
     dfl Locd;                      // L / c as a float pair (pair form)
+    double Loc;                    // L / c (FP64 form)
+    float T2f;                     // T^2 (FP64 form)
     int maxS;                      // largest tile (samples) the shared memory is sized for
     int maxP;                      // most binaries in a tile of this launch (<= kMaxPack)
 };
@@ -123,12 +130,6 @@ enum { MODE_WAVE = 0, MODE_LL = 1, MODE_FILL = 2, MODE_SWAP = 4 };
 __host__ __device__ __forceinline__ int red_doubles(int maxS)
 {
     return 3 * (maxS >> 5) > 8 * kMaxPack ? 3 * (maxS >> 5) : 8 * kMaxPack;
-}
-
-__device__ __forceinline__ double quad_form(const double *e, double x, double y, double z)
-{
-    return e[0] * x * x + e[1] * y * y + e[2] * z * z +
-           2.0 * (e[3] * x * y + e[4] * x * z + e[5] * y * z);
 }
 
 // sin(x) and cos(x) for moderate |x| (the carrier phase reduced to [-pi, pi],
@@ -457,7 +458,12 @@ __device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     const double T = a.T;
     B.b = b;
     B.valid = 1;
-    B.f0 = f0; B.fdot = fdot; B.fddot = fddot; B.phi0 = phi0;
+    B.f0 = f0; B.fdot = fdot; B.fddot = fddot;
+    {
+        // phi0 mod 2 pi: less rounding in the sums it enters (FP64 form)
+        const double k = rint(phi0 * kInvTwoPi);
+        B.phi0 = fma(-k, kTwoPiLo, fma(-k, kTwoPi, phi0));
+    }
     double q = rint(f0 * T);
     // om - 2 pi q/T cancels about seven digits; the two products are rounded
     // separately (no FMA contraction) so the phase slope carries the same
@@ -467,8 +473,9 @@ __device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     B.pifdot = kPi * fdot;
     B.pi3fddot = (1.0 / 3.0 * kPi) * fddot;
     double ci = cos(iota);
-    double s2p, c2p;
-    sincos(2.0 * psi, &s2p, &c2p);
+    double s1p, c1p;
+    sincos(psi, &s1p, &c1p);
+    const double s2p = 2.0 * s1p * c1p, c2p = fma(-2.0 * s1p, s1p, 1.0);
     double Ap = 1.0 + ci * ci, Ac = -2.0 * ci;
     B.DP = make_double2(Ap * c2p, -Ac * s2p);
     B.DC = make_double2(-Ap * s2p, -Ac * c2p);
@@ -479,16 +486,26 @@ __device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     double u[3] = {ct * cp, ct * sp, -st};
     double v[3] = {sp, -cp, 0.0};
     B.k[0] = -st * cp; B.k[1] = -st * sp; B.k[2] = -ct;
-    const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
     if (a.precision == GBX_PAIR) {
         for (int c = 0; c < 3; c++) B.pr.ud[c] = df_from(u[c]);
         for (int c = 0; c < 2; c++) B.pr.vd[c] = df_from(v[c]);
         B.pr.DP = {df_from(B.DP.x), df_from(B.DP.y)};
         B.pr.DC = {df_from(B.DC.x), df_from(B.DC.y)};
     } else {
-        for (int c = 0; c < 6; c++) {
-            B.q.ep[c] = v[ia[c]] * v[ib[c]] - u[ia[c]] * u[ib[c]];
-            B.q.ec[c] = u[ia[c]] * v[ib[c]] + v[ia[c]] * u[ib[c]];
+        // r.e+.r DP + r.ex.r DC = (r.v + i r.u)^2 with its real part times
+        // 1 + cos^2 iota and its imaginary part times 2 cos iota after a turn by
+        // 2 psi: the turn goes into the basis, v' + i u' = (v + i u) e^{i psi}
+        for (int c = 0; c < 3; c++) {
+            B.q.vp[c] = v[c] * c1p - u[c] * s1p;
+            B.q.up[c] = v[c] * s1p + u[c] * c1p;
+        }
+        B.q.ap4 = 0.25 * Ap;
+        B.q.ci = ci;
+        B.q.pf2 = 2.0 * B.pifdot;
+        B.q.p3f3 = 3.0 * B.pi3fddot;
+        for (int c = 0; c < 2; c++) {
+            B.q.kh[c] = rint(B.k[c] * 67108864.0) * (1.0 / 67108864.0);
+            B.q.kl[c] = B.k[c] - B.q.kh[c];
         }
     }
     for (int c = 0; c < 3; c++) {
@@ -651,76 +668,279 @@ __device__ __forceinline__ void slow_unequal_fp64(const Bin &B, double tm, doubl
 }
 
 // ----------------------------------------------------------------------------
-// slow part at one sample (gbgpu.py:399-540 and 348-375)
-// writes fctr2 * {X, Y, Z} (amplitude divided out) into out[0..2]
+// FP64 slow part (gbgpu.py:399-540 and 348-375).  One FP64 warp instruction
+// occupies its scheduler's FP64 unit for 64 cycles (measured), against one
+// cycle for an FP32 one, so the form is bound by the number of FP64
+// instructions and everything below is arranged to need few of them: 381 per
+// sample for the whole likelihood, where every link with its own sincos and
+// the library's sin, sincos and divisions took 754 (10,001 binaries of uneven
+// N: 7.78 -> 4.07 ms; 2,003 windows of N = 512: 1.53 -> 0.84 ms).
 // ----------------------------------------------------------------------------
-template <bool THIRD, bool UNEQ>
-__device__ __forceinline__ void slow_fp64(const Bin &B, int n, int N, double tm, int tdi,
-                                          const double *__restrict__ tab, double fstar,
-                                          const double *psi, const double *vl, double2 out[3])
+// sin x and cos x: table of cos, sin at j pi/128 (tab[j & 255]) and the Taylor
+// series on the remainder |r| <= pi/256 (next terms below 1e-17 and 2e-20),
+// combined by the angle-addition formulas.  pi/128 = C1 + C2 to 106 bits; the
+// FMAs form x - j C1 without an intermediate rounding.  17 FP64 instructions.
+__device__ __forceinline__ double2 turn_tab(double x, const double2 *__restrict__ tab, double &cm, double &sr)
 {
-    double Pc[3][3], r[3][3];
+    constexpr double kInv = 40.74366543152520595683;                // 128/pi
+    constexpr double C1 = 0.024543692606170258;                    // double(pi/128)
+    constexpr double C2 = 9.567553118338697e-19;                    // pi/128 - C1
+    constexpr double kRound = 6755399441055744.0;                   // 1.5 2^52: rounds to integer
+    const double t = fma(x, kInv, kRound);
+    const double jd = t - kRound;
+    const double r = fma(-jd, C2, fma(-jd, C1, x));
+    const double r2 = r * r;
+    sr = fma(r * r2, fma(r2, 1.0 / 120.0, -1.0 / 6.0), r);                      // sin r
+    cm = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);                // cos r - 1
+    return tab[__double2loint(t) & (kScN - 1)];
+}
+
+__device__ __forceinline__ void sincos_tab(double x, const double2 *__restrict__ tab, double &s, double &c)
+{
+    double cm, sr;
+    const double2 cs = turn_tab(x, tab, cm, sr);
+    s = cs.y + fma(cs.y, cm, cs.x * sr);
+    c = cs.x + fma(cs.x, cm, -(cs.y * sr));
+}
+
+// sin(a)/a from its Taylor series in a^2: 5 terms after the first for
+// |a| < 0.16, 7 for |a| < 0.5, 11 for |a| < 1.6 (next terms below 5e-20,
+// 4e-20, 5e-21), sincos_tab beyond.  The last 2, 3 and 5 of them are summed in
+// FP32 (at most 7e-20, 2e-18 and 3e-17 of rounding) and widened on the integer
+// pipe, and the ranges are told apart by the high word.
+__device__ __forceinline__ double sinc_fp64(double a, const double2 *__restrict__ tab)
+{
+    const double x = a * a;
+    const int hx = __double2hiint(x);
+    const float xf = d2f_scaled(x, 0);
+    double p;
+    if (hx < 0x3f9a36e2) {                                  // x < 0.0256
+        p = f2d_bits(fmaf(xf, -1.0f / 39916800.0f, 1.0f / 362880.0f));
+    } else if (hx < 0x3fd00000) {                           // x < 0.25
+        float t = fmaf(xf, -1.0f / 1307674368000.0f, 1.0f / 6227020800.0f);
+        p = fma(x, f2d_bits(fmaf(t, xf, -1.0f / 39916800.0f)), 1.0 / 362880.0);
+    } else if (hx < 0x40047ae1) {                           // x < 2.56
+        float t = fmaf(xf, -1.0f / 25852016738884976640000.0f, 1.0f / 51090942171709440000.0f);
+        t = fmaf(t, xf, -1.0f / 121645100408832000.0f);
+        t = fmaf(t, xf, 1.0f / 355687428096000.0f);
+        p = f2d_bits(fmaf(t, xf, -1.0f / 1307674368000.0f));
+        p = fma(x, p, 1.0 / 6227020800.0);
+        p = fma(x, p, -1.0 / 39916800.0);
+        p = fma(x, p, 1.0 / 362880.0);
+    } else {
+        double s, c;
+        sincos_tab(a, tab, s, c);
+        return s / a;
+    }
+    p = fma(x, p, -1.0 / 5040.0);
+    p = fma(x, p, 1.0 / 120.0);
+    p = fma(x, p, -1.0 / 6.0);
+    return fma(x, p, 1.0);
+}
+
+// 1 / x: the hardware's ~20-bit estimate and two Newton steps (relative error
+// after them ~1 ulp); the division for zero, subnormal, huge and non-finite x.
+__device__ __forceinline__ double recip_fp64(double x)
+{
+    const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+    if (ex - 2u >= 2040u) return 1.0 / x;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(fma(-x, r, 1.0), r, r);
+    return fma(fma(-x, r, 1.0), r, r);
+}
+
+// The general path, used with unequal arms: every link with its own carrier.
+__device__ __forceinline__ void slow_links_fp64(const Bin &B, int n, int N, double tm, int tdi,
+                                             const double *__restrict__ tab, double fstar,
+                                             double2 out[3])
+{
+    double r[3][3];
 #pragma unroll
     for (int s = 0; s < 3; s++)
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            Pc[s][c] = __ldg(tab + (size_t)(3 * s + c) * N + n);
-            r[s][c] = __ldg(tab + (size_t)(9 + 3 * s + c) * N + n);
-        }
-    double kdotr[3], kP[3], xi[3], fonfs[3], kp[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-        kdotr[a] = B.k[0] * r[a][0] + B.k[1] * r[a][1] + B.k[2] * r[a][2];
-#pragma unroll
-    for (int s = 0; s < 3; s++) {
-        kP[s] = B.k[0] * Pc[s][0] + B.k[1] * Pc[s][1] + B.k[2] * Pc[s][2];
-        xi[s] = tm - kP[s];
-        double fi = B.f0 + B.fdot * xi[s] + 0.5 * B.fddot * xi[s] * xi[s];
-        if (THIRD) fi *= 1.0 + vl[s] / kCSI;
-        fonfs[s] = fi / fstar;
-        double argS = B.phi0 + B.om_m_dfa * tm + B.pifdot * xi[s] * xi[s] +
-                      B.pi3fddot * xi[s] * xi[s] * xi[s];
-        if (THIRD) argS += psi[s];
-        kp[s] = B.om * kP[s] - argS;
-    }
+        for (int c = 0; c < 3; c++) r[s][c] = __ldg(tab + (size_t)(9 + 3 * s + c) * N + n);
+    double kdotr[3], fonfs[3], kp[3];
     double2 A[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        double pp = quad_form(B.q.ep, r[a][0], r[a][1], r[a][2]);
-        double cc = quad_form(B.q.ec, r[a][0], r[a][1], r[a][2]);
-        A[a] = make_double2(pp * B.DP.x + cc * B.DC.x, pp * B.DP.y + cc * B.DC.y);
-    }
-    // links (ij, sym arm, spacecraft, sign of kdotr): 12,23,31,21,32,13
-    double2 G[6];
-    const int arm[6] = {0, 1, 2, 0, 1, 2};
-    const int sc[6] = {0, 1, 2, 1, 2, 0};
-    const double sg[6] = {1.0, 1.0, 1.0, -1.0, -1.0, -1.0};
-    if constexpr (UNEQ) {
-        slow_unequal_fp64(B, tm, fstar, r, kdotr, fonfs, kp, A, tdi, out);
-        return;
+        kdotr[a] = B.k[0] * r[a][0] + B.k[1] * r[a][1] + B.k[2] * r[a][2];
+        const double ru = B.q.up[0] * r[a][0] + B.q.up[1] * r[a][1] + B.q.up[2] * r[a][2];
+        const double rv = B.q.vp[0] * r[a][0] + B.q.vp[1] * r[a][1] + B.q.vp[2] * r[a][2];
+        A[a] = make_double2(4.0 * B.q.ap4 * (rv * rv - ru * ru), 4.0 * B.q.ci * ru * rv);
     }
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
-        double arg = 0.5 * fonfs[sc[q]] * (1.0 + sg[q] * kdotr[arm[q]]);
-        double sn, cs;
-        sincos(arg + kp[sc[q]], &sn, &cs);
-        double amp = 0.25 * sin(arg) / arg;
-        double2 e = make_double2(amp * cs, -amp * sn);
-        G[q] = cmul(e, A[arm[q]]);
+    for (int s = 0; s < 3; s++) {
+        double kP = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; c++) kP = fma(B.k[c], __ldg(tab + (size_t)(3 * s + c) * N + n), kP);
+        const double xi = tm - kP;
+        fonfs[s] = (B.f0 + B.fdot * xi + 0.5 * B.fddot * xi * xi) / fstar;
+        kp[s] = B.om * kP - (B.phi0 + B.om_m_dfa * tm + B.pifdot * xi * xi + B.pi3fddot * xi * xi * xi);
     }
-    double f = B.f0 + B.fdot * tm + 0.5 * B.fddot * tm * tm;
-    double omL = f / fstar;
-    double so, co;
-    sincos(omL, &so, &co);
-    double2 fc = make_double2(co, -so);
-    double2 fc2 = make_double2(4.0 * omL * so * co, -4.0 * omL * so * so);
-    // X = G21 - G31 + (G12 - G13) fc, cyclic (gbgpu.py:370-372)
-    double2 X = cadd(csub(G[3], G[2]), cmul(csub(G[0], G[5]), fc));
-    double2 Y = cadd(csub(G[4], G[0]), cmul(csub(G[1], G[3]), fc));
-    double2 Z = cadd(csub(G[5], G[1]), cmul(csub(G[2], G[4]), fc));
-    out[0] = cmul(fc2, X);
-    out[1] = cmul(fc2, Y);
-    out[2] = cmul(fc2, Z);
+    slow_unequal_fp64(B, tm, fstar, r, kdotr, fonfs, kp, A, tdi, out);
+}
+
+// Equal arms: A and E (AE, formed before the transform) or X, Y, Z at one
+// sample, amplitude divided out.
+//
+// With L/c = 1/(2 pi f*), arm a = 12, 23, 31 from spacecraft a to a + 1 and
+// k.P_s/c - k.P_1/c = del_s = (L/c) {0, k.r_12, -k.r_31}, spacecraft s has the
+// carrier phase and f/f*
+//   phi_s = phi_1 + del_s (W0 - del_s W1),  fo_s = (L/c) (W0 - 2 del_s W1),
+//   W0 = 2 pi f(xi_1), W1 = pi fdot(xi_1)
+// (exact in fdot; left out are pi/3 fddot del^3 < 600 s^3 fddot radians and
+// its share of fo_s).  The two links of an arm carry the angles
+// th = a+ + phi_a and th + d with d = -(L/c)^2 W1 k.r_a (the (L/c) k.r W0
+// terms cancel exactly), so one sincos per arm is enough.  With h = omL/2,
+// S+- = sin(a+-)/a+-, p = S+ + S-, m = S+ - S- and
+// z_a = A_a e^{-i (th + d/2 + 3h)}, the TDI combination
+// fc2 (G21 - G31 + (G12 - G13) fc) (gbgpu.py:362-372) becomes, with
+//   U = [p cos h cos(d/2) + i m cos h sin(d/2)] z,
+//   V = [m sin h cos(d/2) + i p sin h sin(d/2)] z,
+//   X = 4 omL sin(omL) [(U_1 - i V_1) - (U_3 + i V_3)]  (Y, Z cyclic).
+// d is ~1e-13 rad: its part of U and V is added in FP32 and widened on the
+// integer pipe (no FP64 instruction), in FP64 from 1e-9 on.
+// THIRD: psi_s is taken off phi_s and fo_s grows by the factor 1 + v_s/c, which
+// d follows (|d| ~ 1e-5; the sincos of d/2 itself above 1e-4).
+template <bool THIRD, bool AE>
+__device__ __forceinline__ void slow_fp64(const Bin &B, int n, int N, double tm,
+                                          const double *__restrict__ tab, double Loc,
+                                          const double2 *__restrict__ sct, bool chirp,
+                                          const double *psi, const double *vl, double2 out[3])
+{
+    double kr[3], ru[3], rv[3];
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        const double r0 = __ldg(tab + (size_t)(9 + 3 * a) * N + n);
+        const double r1 = __ldg(tab + (size_t)(10 + 3 * a) * N + n);
+        const double r2 = __ldg(tab + (size_t)(11 + 3 * a) * N + n);
+        kr[a] = fma(B.k[2], r2, fma(B.k[1], r1, B.k[0] * r0));
+        ru[a] = fma(B.q.up[2], r2, fma(B.q.up[1], r1, B.q.up[0] * r0));
+        rv[a] = fma(B.q.vp[2], r2, fma(B.q.vp[1], r1, B.q.vp[0] * r0));
+    }
+    // r_31 = -(r_12 + r_23): differences of the same positions
+    kr[2] = -(kr[0] + kr[1]);
+    ru[2] = -(ru[0] + ru[1]);
+    rv[2] = -(rv[0] + rv[1]);
+    // k.P_1/c = s + r, s exact: multiples of 2^-43 below 2^10 (2^-26 times 2^-17)
+    const double P0 = __ldg(tab + n), P1 = __ldg(tab + (size_t)N + n);
+    const double H0 = __ldg(tab + (size_t)36 * N + n), H1 = __ldg(tab + (size_t)37 * N + n);
+    const double L0 = __ldg(tab + (size_t)38 * N + n), L1 = __ldg(tab + (size_t)39 * N + n);
+    const double s = fma(B.q.kh[1], H1, B.q.kh[0] * H0);
+    const double r = fma(B.q.kh[1], L1, fma(B.q.kh[0], L0, fma(B.q.kl[1], P1,
+                         fma(B.q.kl[0], P0, B.k[2] * __ldg(tab + (size_t)2 * N + n)))));
+    const double xi = tm - (s + r);
+    const double fx = B.pi3fddot * xi;
+    // The phase of spacecraft 1, om kP - (om - df) tm - phi0 - pf xi^2 with
+    // pf = pi fdot + pi/3 fddot xi, is one term of every link's angle, so its
+    // rounding does not average out over the links as that of separately
+    // formed phases does: the large products keep their rounding errors
+    // (lo), and om kP is reduced mod 2 pi before the sum.
+    constexpr double kRound = 6755399441055744.0;
+    const double pf = B.pifdot + fx, xi2 = xi * xi;
+    double big = B.om * s, lo = fma(B.om, r, fma(B.om, s, -big));
+    double arg = fma(B.om_m_dfa, tm, B.phi0);
+    if (chirp) {
+        // pf xi^2 above a fraction of a radian somewhere: with the error of xi,
+        // its square and the product, and TwoSum into the large part
+        const double g = pf * xi2;
+        const double c2 = fma(xi + xi, ((tm - xi) - s) - r, fma(xi, xi, -xi2));
+        const double gl = fma(pf, c2, fma(pf, xi2, -g));
+        const double S = big - g, bb = S - big;
+        lo += ((big - (S - bb)) - (g + bb)) - gl;
+        big = S;
+    } else {
+        arg = fma(pf, xi2, arg);
+    }
+    const double turns = fma(big, kInvTwoPi, kRound) - kRound;
+    double ph[3], fo[3];
+    ph[0] = fma(-turns, kTwoPi, big) - arg;
+    lo = fma(-turns, kTwoPiLo, lo);
+    const double W1 = fma(3.0, fx, B.pifdot);
+    const double W0 = fma(xi, W1 + B.pifdot, B.om);
+    const double hLoc = 0.5 * Loc;
+    const double h = hLoc * fma(tm, fma(B.q.p3f3, tm, B.q.pf2), B.om);        // omL/2
+    ph[0] += fma(3.0, h, lo);
+    // fo: half of f/f* from here on
+    fo[0] = hLoc * W0;
+    const double dw = -Loc * W1;
+    const double del1 = Loc * kr[0], del2 = -Loc * kr[2];
+    fo[1] = fma(dw, del1, fo[0]);
+    fo[2] = fma(dw, del2, fo[0]);
+    ph[1] = fma(del1, fma(-del1, W1, W0), ph[0]);
+    ph[2] = fma(del2, fma(-del2, W1, W0), ph[0]);
+    const double dd = hLoc * dw;                                // d/2 = dd k.r
+    double dv[3];
+    if (THIRD) {
+#pragma unroll
+        for (int s = 0; s < 3; s++) {
+            ph[s] -= psi[s];
+            dv[s] = fo[s] * (vl[s] * (1.0 / kCSI));
+            fo[s] += dv[s];
+        }
+    }
+    // |d| < 1e-9 everywhere (|k.r| <= 1): high word of dd below that of 5e-10
+    const bool tiny = !THIRD && (__double2hiint(dd) & 0x7fffffff) < 0x3e012e0b;
+    double sh, ch;
+    sincos_tab(h, sct, sh, ch);
+    double2 U[3], V[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const int s2 = a == 2 ? 0 : a + 1;
+        const double ap = fma(fo[a], kr[a], fo[a]), am = fma(-fo[s2], kr[a], fo[s2]);
+        const double Sp = sinc_fp64(ap, sct), Sm = sinc_fp64(am, sct);
+        double d2 = dd * kr[a];
+        if (THIRD)
+            d2 += 0.5 * ((psi[a] - psi[s2]) + (fma(-dv[s2], kr[a], dv[s2]) - fma(dv[a], kr[a], dv[a])));
+        const double Ar = B.q.ap4 * fma(rv[a], rv[a], -(ru[a] * ru[a]));
+        const double Ai = B.q.ci * (ru[a] * rv[a]);
+        // z = (A e^{-i theta_tab}) e^{-i r}
+        double cm, sr;
+        const double2 t = turn_tab(ph[a] + (ap + d2), sct, cm, sr);
+        const double2 w = make_double2(fma(Ai, t.y, Ar * t.x), fma(Ai, t.x, -(Ar * t.y)));
+        const double2 z = make_double2(fma(w.x, cm, fma(w.y, sr, w.x)), fma(w.y, cm, fma(-w.x, sr, w.y)));
+        const double p = Sp + Sm, m = Sp - Sm;
+        if (tiny) {
+            const float d2f = d2f_scaled(d2, 0);
+            const float e2 = d2f_scaled(m, 0) * d2f_scaled(ch, 0) * d2f;
+            const float e1 = d2f_scaled(p, 0) * d2f_scaled(sh, 0) * d2f;
+            const float zx = d2f_scaled(z.x, 0), zy = d2f_scaled(z.y, 0);
+            const double pc = p * ch, ms = m * sh;
+            U[a] = make_double2(fma(pc, z.x, f2d_bits(-e2 * zy)), fma(pc, z.y, f2d_bits(e2 * zx)));
+            V[a] = make_double2(fma(ms, z.x, f2d_bits(-e1 * zy)), fma(ms, z.y, f2d_bits(e1 * zx)));
+        } else {
+            double sd, cd;
+            if (fabs(d2) < 0.5e-4) {
+                const double e = -0.5 * d2 * d2;
+                cd = 1.0 + e;
+                sd = d2 * fma(1.0 / 3.0, e, 1.0);
+            } else {
+                sincos_tab(d2, sct, sd, cd);
+            }
+            const double pc = p * ch * cd, ms = m * sh * cd, e2 = m * ch * sd, e1 = p * sh * sd;
+            U[a] = make_double2(fma(pc, z.x, -(e2 * z.y)), fma(pc, z.y, e2 * z.x));
+            V[a] = make_double2(fma(ms, z.x, -(e1 * z.y)), fma(ms, z.y, e1 * z.x));
+        }
+    }
+    const double g4 = 16.0 * h * sh * ch;                       // 4 omL sin(omL)
+    if constexpr (AE) {
+        // Z - X = 2 U_3 - (U_1 + U_2) + i (V_1 - V_2),
+        // X - 2Y + Z = 3 (U_1 - U_2) + i (V_1 + V_2 - 2 V_3)
+        const double gA = 0.70710678118654752440 * g4, gE = 0.40824829046386301637 * g4;
+        const double2 us = cadd(U[0], U[1]), ud = csub(U[0], U[1]);
+        const double2 vs = cadd(V[0], V[1]), vd = csub(V[0], V[1]);
+        out[0] = make_double2(gA * (fma(2.0, U[2].x, -us.x) - vd.y), gA * (fma(2.0, U[2].y, -us.y) + vd.x));
+        out[1] = make_double2(gE * fma(3.0, ud.x, -fma(-2.0, V[2].y, vs.y)),
+                              gE * fma(3.0, ud.y, fma(-2.0, V[2].x, vs.x)));
+    } else {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const int e = c == 0 ? 2 : c - 1;                   // X: 1, 3; Y: 2, 1; Z: 3, 2
+            out[c] = make_double2(g4 * ((U[c].x - U[e].x) + (V[c].y + V[e].y)),
+                                  g4 * ((U[c].y - U[e].y) - (V[c].x + V[e].x)));
+        }
+    }
 }
 
 // Spacecraft 1's delay k . P_1 / c at sample n as a float pair, from the
@@ -1021,6 +1241,118 @@ __device__ __forceinline__ void fft_dif(typename C2<R>::T *buf, int nsub, int lg
     __syncthreads();
 }
 
+// FP64: the same transform with fewer FP64 instructions (each costs 64 cycles
+// of its scheduler, so nothing else matters).  A register pass takes its 2, 4
+// or 8 elements as one small DFT whose inner factors are 1, -i and
+// (+-1 - i)/sqrt2, and multiplies output k once by W^(r k): 84 instructions
+// per 8 elements instead of 96, 28 per 4 instead of 32.
+template <int RB>
+__device__ __forceinline__ void fft_reg_pass_d(double2 *buf, int nsub, int lg, int hl)
+{
+    constexpr int M = 1 << RB;
+    const int q = hl - RB + 1;
+    const int groups = nsub << (lg - RB);
+    const int ts = kTwN >> (hl + 1);
+    for (int g = threadIdx.x; g < groups; g += kBlock) {
+        const int a = g >> (lg - RB);
+        const int rem = g & ((1 << (lg - RB)) - 1);
+        const int blk = rem >> q;
+        const int r = rem & ((1 << q) - 1);
+        double2 *sub = buf + ((size_t)a << lg);
+        const int p0 = (blk << (hl + 1)) + r;
+        double2 x[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) x[m] = sub[swz(p0 + (m << q), lg)];
+#pragma unroll
+        for (int j = 0; j < RB; j++) {
+            const int dm = M >> (j + 1);
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                if (m & dm) continue;
+                const double2 u = x[m], t = csub(u, x[m + dm]);
+                x[m] = cadd(u, x[m + dm]);
+                // times exp(-i pi e / 4)
+                const int e = (m & (dm - 1)) * (4 / dm);
+                constexpr double h = 0.70710678118654752440;
+                if (e == 0) x[m + dm] = t;
+                else if (e == 2) x[m + dm] = make_double2(t.y, -t.x);
+                else if (e == 1) x[m + dm] = make_double2((t.x + t.y) * h, (t.y - t.x) * h);
+                else x[m + dm] = make_double2((t.y - t.x) * h, -(t.x + t.y) * h);
+            }
+        }
+        sub[swz(p0, lg)] = x[0];
+#pragma unroll
+        for (int m = 1; m < M; m++) {
+            // register m holds output k = bitrev(m); W^(r k), the table's half
+            // period continued by its sign
+            const int k = RB == 1 ? 1 : RB == 2 ? ((m & 1) << 1) | (m >> 1)
+                                                : ((m & 1) << 2) | (m & 2) | (m >> 2);
+            const int idx = r * k * ts;
+            double2 w = tw<double>(idx & (kTwN / 2 - 1));
+            if (idx & (kTwN / 2)) w = make_double2(-w.x, -w.y);
+            sub[swz(p0 + (m << q), lg)] = cmul(x[m], w);
+        }
+    }
+}
+
+// last five stages on 32-element blocks, one block per half-warp with two
+// elements per lane (as fft_dif_pair: the lane trades one element with lane
+// l ^ h before each stage, so no butterfly is computed twice): 16 FP64
+// instructions per element instead of 22
+__device__ __forceinline__ void fft_dif_d(double2 *buf, int nsub, int lg)
+{
+    int hl = lg - 1;
+    while (hl >= 5) {
+        const int rb = (hl - 4) >= 3 ? 3 : (hl - 4);
+        if (rb == 3) fft_reg_pass_d<3>(buf, nsub, lg, hl);
+        else if (rb == 2) fft_reg_pass_d<2>(buf, nsub, lg, hl);
+        else fft_reg_pass_d<1>(buf, nsub, lg, hl);
+        hl -= rb;
+        __syncthreads();
+    }
+    const int lane = threadIdx.x & 31;
+    const int l = lane & 15;
+    double2 w[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int hh = 4 - k;
+        w[k] = tw<double>((l & ((1 << hh) - 1)) * (kTwN >> (hh + 1)));
+    }
+    const int blocks = (nsub << lg) >> 5;
+    const int npairs = (blocks + 1) >> 1;
+    for (int c = threadIdx.x >> 5; c < npairs; c += kBlock >> 5) {
+        const int blk = 2 * c + (lane >> 4);
+        const bool live = blk < blocks;
+        const int e0 = (live ? blk : blocks - 1) << 5;   // a spare half-warp repeats the last block
+        double2 *sub = buf + ((e0 >> lg) << lg);
+        const int off = e0 & ((1 << lg) - 1);
+        double2 u = sub[swz(off + l, lg)], v = sub[swz(off + l + 16, lg)];
+        {
+            const double2 t = csub(u, v);
+            u = cadd(u, v);
+            v = cmul(t, w[0]);
+        }
+#pragma unroll
+        for (int k = 1; k < 5; k++) {
+            const int h = 16 >> k;
+            const bool bit = (l & h) != 0;
+            const double2 rcv = shfl_c<double>(bit ? u : v, h);
+            if (bit) u = rcv;
+            else v = rcv;
+            const double2 t = csub(u, v);
+            u = cadd(u, v);
+            if (k < 3) v = cmul(t, w[k]);
+            else if (k == 3) v = (l & 1) ? make_double2(t.y, -t.x) : t;
+            else v = t;
+        }
+        if (live) {
+            sub[swz(off + 2 * l, lg)] = u;
+            sub[swz(off + 2 * l + 1, lg)] = v;
+        }
+    }
+    __syncthreads();
+}
+
 // ----------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------
@@ -1225,11 +1557,16 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
     extern __shared__ __align__(16) unsigned char smem[];
     Bin *bins = reinterpret_cast<Bin *>(smem);
     double *red = reinterpret_cast<double *>(smem + sizeof(Bin) * K.maxP);
-    V *buf = reinterpret_cast<V *>(smem + sizeof(Bin) * K.maxP + sizeof(double) * red_doubles(K.maxS));
+    // FP64 form: the sin/cos table lies between the reduction scratch and buf
+    constexpr int kSc = sizeof(R) == 8 ? kScN : 0;
+    double2 *sct = reinterpret_cast<double2 *>(smem + sizeof(Bin) * K.maxP +
+                                               sizeof(double) * red_doubles(K.maxS));
+    V *buf = reinterpret_cast<V *>(sct + kSc);
     __shared__ int s_tile;
 
     const gbx_wave_args &a = K.a;
     const int tid = threadIdx.x;
+    for (int k = tid; k < kSc; k += kBlock) sct[k] = g_sc_d[k];
     const int ntiles = a.tiles ? a.ntiles : (a.num_bin + K.P - 1) / K.P;
     const double fstar = K.fstar;
     const float Loc = (float)(1.0 / (kTwoPi * fstar));         // L / c
@@ -1311,7 +1648,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
         for (int m = tid; m < S; m += kBlock) {
             const int p = m >> lg, n = m & (N - 1);
             const Bin &B = bins[p];
-            const double tm = (double)n * step;
+            const double tm = f2d_bits((float)n) * step;
             double ps[3] = {0.0, 0.0, 0.0};
             dfl psf[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
             R vv[3] = {0, 0, 0};
@@ -1328,16 +1665,17 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                 // nothing of this binary reaches the outputs (bad index, or a
                 // zero-amplitude fill): skip the slow part
                 o[0] = o[1] = o[2] = V{0, 0};
+            } else if constexpr (sizeof(R) == 8 && !UNEQ) {
+                const bool chirp = fmaf(fabsf(B.fddotf), (float)a.T, fabsf(B.fdotf)) * K.T2f > 0.3f;
+                slow_fp64<THIRD, NCH == 2>(B, n, N, tm, tab, K.Loc, sct, chirp, ps, vv, o);
             } else if constexpr (sizeof(R) == 8) {
-                double vd[3] = {(double)vv[0], (double)vv[1], (double)vv[2]};
-                slow_fp64<THIRD, UNEQ>(B, n, N, tm, a.tdi2, tab, fstar, ps, vd, reinterpret_cast<double2 *>(o));
+                slow_links_fp64(B, n, N, tm, a.tdi2, tab, fstar, o);
             } else {
-                float vf[3] = {(float)vv[0], (float)vv[1], (float)vv[2]};
-                slow_mixed<THIRD>(B, n, N, stepd, Loc, tab, psf, vf, reinterpret_cast<float2 *>(o));
+                slow_mixed<THIRD>(B, n, N, stepd, Loc, tab, psf, vv, o);
             }
-            if constexpr (NCH == 3) {
+            if constexpr (NCH == 3 || (sizeof(R) == 8 && !UNEQ)) {
 #pragma unroll
-                for (int c = 0; c < 3; c++) buf[(p * 3 + c) * N + swz(n, lg)] = o[c];
+                for (int c = 0; c < NCH; c++) buf[(p * NCH + c) * N + swz(n, lg)] = o[c];
             } else {
                 // A = (Z - X)/sqrt2, E = (X - 2Y + Z)/sqrt6 (utility.py:24-38) formed
                 // before the transform: the FFT is linear, so two transforms suffice
@@ -1348,7 +1686,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
         }
         __syncthreads();
 
-        fft_dif<R>(buf, NCH * cnt, lg);
+        if constexpr (sizeof(R) == 8) fft_dif_d(buf, NCH * cnt, lg);
+        else fft_dif<R>(buf, NCH * cnt, lg);
 
         // ------------------------------------------------------------ epilogue
         if (MODE == MODE_WAVE) {
@@ -1432,7 +1771,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                         const double SA = __ldg(K.A_psd + jn), SE = __ldg(K.E_psd + jn);
                         Acc wA, wE, aR, aI, eR, eI;
                         if constexpr (sizeof(R) == 8) {
-                            wA = 1.0 / SA; wE = 1.0 / SE;
+                            wA = recip_fp64(SA);
+                            wE = K.A_psd == K.E_psd ? wA : recip_fp64(SE);
                             aR = dA.x; aI = dA.y; eR = dE.x; eI = dE.y;
                         } else {
                             wA = __frcp_rn(d2f_scaled(SA, Bn.eS));
@@ -1595,12 +1935,10 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                         if (samepsd) {
                             const double S = __ldg(K.A_psd + jn);
                             if constexpr (sizeof(R) == 8) {
-                                const double2 hA = cmul(make_double2(tA.x, tA.y), B.scale);
-                                const double2 hE = cmul(make_double2(tE.x, tE.y), B.scale);
-                                const double w = 1.0 / S;
-                                sr += ((dA.x * hA.x + dA.y * hA.y) + (dE.x * hE.x + dE.y * hE.y)) * w;
-                                si += ((dA.x * hA.y - dA.y * hA.x) + (dE.x * hE.y - dE.y * hE.x)) * w;
-                                sh += ((hA.x * hA.x + hA.y * hA.y) + (hE.x * hE.x + hE.y * hE.y)) * w;
+                                const double w = recip_fp64(S);
+                                sr = fma((dA.x * tA.x + dA.y * tA.y) + (dE.x * tE.x + dE.y * tE.y), w, sr);
+                                si = fma((dA.x * tA.y - dA.y * tA.x) + (dE.x * tE.y - dE.y * tE.x), w, si);
+                                sh = fma((tA.x * tA.x + tA.y * tA.y) + (tE.x * tE.x + tE.y * tE.y), w, sh);
                             } else {
                                 const float w = __frcp_rn(d2f_scaled(S, B.eS));
                                 const float aR = d2f_scaled(dA.x, B.eD), aI = d2f_scaled(dA.y, B.eD);
@@ -1613,13 +1951,11 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                         }
                         const double SA = __ldg(K.A_psd + jn), SE = __ldg(K.E_psd + jn);
                         if constexpr (sizeof(R) == 8) {
-                            double2 hA = cmul(make_double2(tA.x, tA.y), B.scale);
-                            double2 hE = cmul(make_double2(tE.x, tE.y), B.scale);
-                            const double wA = 1.0 / SA, wE = 1.0 / SE;
+                            const double wA = recip_fp64(SA), wE = recip_fp64(SE);
                             // conj(d) h / S  (gbgpu_utils.cu:172-178)
-                            sr += (dA.x * hA.x + dA.y * hA.y) * wA + (dE.x * hE.x + dE.y * hE.y) * wE;
-                            si += (dA.x * hA.y - dA.y * hA.x) * wA + (dE.x * hE.y - dE.y * hE.x) * wE;
-                            sh += (hA.x * hA.x + hA.y * hA.y) * wA + (hE.x * hE.x + hE.y * hE.y) * wE;
+                            sr += (dA.x * tA.x + dA.y * tA.y) * wA + (dE.x * tE.x + dE.y * tE.y) * wE;
+                            si += (dA.x * tA.y - dA.y * tA.x) * wA + (dE.x * tE.y - dE.y * tE.x) * wE;
+                            sh += (tA.x * tA.x + tA.y * tA.y) * wA + (tE.x * tE.x + tE.y * tE.y) * wE;
                         } else {
                             const float2 hA = tA, hE = tE;
                             const float wA = __frcp_rn(d2f_scaled(SA, B.eS));
@@ -1697,17 +2033,12 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                 const double tr = tsum[3 * tid], ti = tsum[3 * tid + 1], th = tsum[3 * tid + 2];
                 const double s4 = 4.0 * K.df;
                 double2 dh, hv;
-                if constexpr (sizeof(R) == 8) {
-                    dh = make_double2(s4 * tr, s4 * ti);
-                    hv = make_double2(s4 * th, 0.0);
-                } else {
-                    // undo the power-of-two scalings and apply amp * 0.5T/N [* tdi2]
-                    const double cd = s4 * exp2_int(B.eS - B.eD);
-                    const double ch = s4 * exp2_int(B.eS) *
-                                      (B.scale.x * B.scale.x + B.scale.y * B.scale.y);
-                    dh = cmul(make_double2(cd * tr, cd * ti), B.scale);
-                    hv = make_double2(ch * th, 0.0);
-                }
+                // undo the mixed form's power-of-two scalings and apply amp * 0.5T/N [* tdi2]
+                const double cd = sizeof(R) == 8 ? s4 : s4 * exp2_int(B.eS - B.eD);
+                const double ch = (sizeof(R) == 8 ? s4 : s4 * exp2_int(B.eS)) *
+                                  (B.scale.x * B.scale.x + B.scale.y * B.scale.y);
+                dh = cmul(make_double2(cd * tr, cd * ti), B.scale);
+                hv = make_double2(ch * th, 0.0);
                 if (!B.valid) {
                     dh = make_double2(0.0, 0.0);
                     hv = make_double2(0.0, 0.0);
@@ -1779,7 +2110,8 @@ constexpr int kPairMaxLog2N = 12;  // pair form: N <= 4096 (two 16-byte channels
 // FP64 scratch and keep psi and v_LOS after them
 static size_t smem_bytes(int prec, bool third, int maxS, int nch, int maxP)
 {
-    size_t head = sizeof(Bin) * (size_t)maxP + sizeof(double) * (size_t)red_doubles(maxS);
+    size_t head = sizeof(Bin) * (size_t)maxP + sizeof(double) * (size_t)red_doubles(maxS) +
+                  (prec == GBX_FP64 ? kScN * sizeof(double2) : 0);
     size_t rc = prec == GBX_FP64 ? sizeof(double2) : sizeof(float2);
     size_t r = prec == GBX_FP64 ? sizeof(double) : sizeof(float);
     size_t s = head + (third ? 3 : nch) * (size_t)maxS * rc;
@@ -1929,6 +2261,8 @@ static KParams base_params(const gbx_wave_args *a)
     K.fstar = kCSI / (a->armlength * 2.0 * kPi);
     for (int k = 0; k <= GBX_MAX_LOG2N; k++) K.stepd[k] = df_from(ldexp(a->T, -k));
     K.Locd = df_from(a->armlength / kCSI);
+    K.Loc = a->armlength / kCSI;
+    K.T2f = (float)(a->T * a->T);
     K.P = a->tiles == nullptr ? tile_pack(a->tile, 31 - __builtin_clz((unsigned)a->N), 1) : 1;
     return K;
 }

@@ -170,7 +170,8 @@ int gbx_fill_global_det(void *A_glob, void *E_glob, const void *A_template,
  * reads.  `table` must hold gbx_orbit_table_bytes(N) bytes, 16-byte aligned.
  * Layout (rows of N, sample n fastest): 18 FP64 rows P_s/c, r_12, r_23,
  * r_31; then 36 FP32 rows: r (9), P_s/c as float pairs (9 heads, 9 tails),
- * r's tails (9).
+ * r's tails (9); then 4 FP64 rows: x and y of P_1/c rounded to 2^-17 s, and
+ * what the rounding took off.
  */
 size_t gbx_orbit_table_bytes(int N);
 int gbx_orbit_table(void *table, const double *sc_pos, int N, double armlength,
