@@ -71,10 +71,17 @@ struct __align__(16) Bin {
     };
     double2 DP, DC;                // polarisation factors divided by amp
     double2 scale;                 // amp * 0.5 T / N [* tdi2 factor]
-    double A2, varpi, e2;          // third body (FP64 form)
     union { double n2; dfl n2d; }; // n2 [rad/s]: FP64 form / float pair (mixed form)
     union { double T2; dfl T2d; }; // T2 [s], likewise
-    float kf[3], uf[3], vf[3];      // k, u, v in FP32 (mixed form; r.e+.r = (r.v)^2 - (r.u)^2)
+    union {
+        struct {
+            float kf[3], uf[3], vf[3];   // k, u, v in FP32 (mixed form; r.e+.r = (r.v)^2 - (r.u)^2)
+        };
+        struct {
+            // FP64 form: v_LOS = (ka sin u + kb cos u)/(1 - eD cos u) + kc
+            double e2, eD, ka, kb, kc;
+        } kep;
+    };
     float2 DPf, DCf;
     float f0f, fdotf, fddotf;
     float w0h, w0l, w1, w2;        // f(t)/fstar = (w0h + w0l) + w1 t + w2 t^2 (w0 split hi/lo)
@@ -281,62 +288,12 @@ __device__ __forceinline__ double2 f2d(float2 v)
 }
 
 // ----------------------------------------------------------------------------
-// third body: line-of-sight velocity (gbgpu/thirdbody.py:228-380)
+// third body: line-of-sight velocity (gbgpu/thirdbody.py:228-380); the FP64
+// form's vlos3_fp64 stands with its pre-pass below
 // ----------------------------------------------------------------------------
-__device__ double vlos_fp64(double t, const Bin &B)
-{
-    // Kepler inverse exactly as gbgpu/thirdbody.py:243-320
-    double l = B.n2 * (t - B.T2);
-    double e = B.e2;
-    bool neg = l < 0.0;
-    l = fabs(l);
-    bool over2pi = l > 2.0 * kPi;
-    double mult = 0.0;
-    if (over2pi) {
-        mult = floor(l / (2.0 * kPi));
-        l -= mult * 2.0 * kPi;
-    }
-    bool overpi = l > kPi;
-    if (overpi) l = 2.0 * kPi - l;
-    double alpha = (1.0 - e) / (4.0 * e + 0.5);
-    double beta = 0.5 * l / (4.0 * e + 0.5);
-    double z = sqrt(beta * beta + alpha * alpha * alpha);
-    z = neg ? beta - z : beta + z;
-    z = (z < 0.0) ? -pow(-z, 1.0 / 3.0) : pow(z, 1.0 / 3.0);
-    double s = z - alpha / z;
-    double w = s - 0.078 * s * s * s * s * s / (1.0 + e);
-    double u0 = l + e * (3.0 * w - 4.0 * w * w * w);
-    double su0, cu0;
-    sincos(u0, &su0, &cu0);
-    double f = u0 - e * su0 - l;
-    double f1 = 1.0 - e * cu0;
-    double f2 = u0 - f - l;
-    double f3 = 1.0 - f1;
-    double f4 = -f2;
-    f2 *= 0.5;
-    f3 *= 0.166666666666667;
-    f4 *= 0.0416666666666667;
-    double u1 = -f / f1;
-    double u2 = -f / (f1 + f2 * u1);
-    double u3 = -f / (f1 + f2 * u2 + f3 * u2 * u2);
-    double u4 = -f / (f1 + f2 * u3 + f3 * u3 * u3 + f4 * u3 * u3 * u3);
-    double u = u0 + u4;
-    if (overpi) u = 2.0 * kPi - u;
-    if (over2pi) u = 2.0 * kPi * mult + u;
-    if (neg) u = -u;
-    // true anomaly (gbgpu/thirdbody.py:339-350)
-    if (e > 1e-6) {
-        double bt = (1.0 - sqrt(1.0 - e * e)) / e;
-        double su, cu;
-        sincos(u, &su, &cu);
-        u += 2.0 * atan2(bt * su, 1.0 - bt * cu);
-    }
-    return B.A2 * (sin(u + B.varpi) + e * sin(B.varpi));
-}
-
-// Same model with the Kepler solve in FP32: eccentric anomaly u for a mean
-// anomaly l in [0, pi] (Mikkola's starter and a fourth-order Newton step, as
-// the FP64 form).
+// Kepler's equation in FP32: eccentric anomaly u for a mean
+// anomaly l in [0, pi] (Mikkola's starter and a fourth-order Newton step,
+// gbgpu/thirdbody.py:243-320).
 __device__ __forceinline__ float kepler_solve_f(float l, float e)
 {
     float alpha = (1.0f - e) / (4.0f * e + 0.5f);
@@ -509,9 +466,11 @@ __device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
         }
     }
     for (int c = 0; c < 3; c++) {
-        B.kf[c] = (float)B.k[c];
-        B.uf[c] = (float)u[c];
-        B.vf[c] = (float)v[c];
+        if (a.precision != GBX_FP64) {
+            B.kf[c] = (float)B.k[c];
+            B.uf[c] = (float)u[c];
+            B.vf[c] = (float)v[c];
+        }
         B.kd[c] = df_from(B.k[c]);
     }
     B.omd = df_from(B.om);
@@ -553,23 +512,37 @@ __device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     }
     B.scale = sc;
     if (a.nparams >= 14) {
-        B.A2 = p[9 * nb + b];
-        B.varpi = p[10 * nb + b];
-        B.e2 = p[11 * nb + b];
+        const double A2 = p[9 * nb + b], varpi = p[10 * nb + b], e2 = p[11 * nb + b];
         double P2 = p[12 * nb + b];
         const double n2 = 2.0 * kPi / (P2 * a.year), T2 = p[13 * nb + b] * a.year;
         if (a.precision == GBX_FP64) {
             B.n2 = n2;
             B.T2 = T2;
+            // A2 [sin(phi + varpi) + e sin varpi] with the true anomaly
+            // phi = u + 2 arg(1 - bt e^{-iu}), bt = (1 - sqrt(1 - e^2))/e
+            // (gbgpu/thirdbody.py:339-380), that is sin phi = sq sin u/(1 - eD cos u),
+            // cos phi = (cos u - eD)/(1 - eD cos u) with eD = 2 bt/(1 + bt^2) and
+            // sq = (1 - bt^2)/(1 + bt^2): eD is e up to bt's rounding, which
+            // reaches 1e-10 for small e and is kept as the model has it.  Below
+            // e = 1e-6 the model takes phi = u: bt = 0.
+            double sv, cv;
+            sincos(varpi, &sv, &cv);
+            const double bt = e2 > 1e-6 ? (1.0 - sqrt(1.0 - e2 * e2)) / e2 : 0.0;
+            const double ib = 1.0 / fma(bt, bt, 1.0), eD = 2.0 * bt * ib, sq = (1.0 - bt) * (1.0 + bt) * ib;
+            B.kep.e2 = e2;
+            B.kep.eD = eD;
+            B.kep.ka = A2 * (sq * cv);
+            B.kep.kb = A2 * (sq * sq * sv);                       // 1 - eD^2 = sq^2
+            B.kep.kc = A2 * ((e2 - eD) * sv);
         } else {
             B.n2d = df_from(n2);
             B.T2d = df_from(T2);
         }
-        B.A2f = (float)B.A2;
-        B.e2f = (float)B.e2;
-        double vr = B.varpi - 2.0 * kPi * floor(B.varpi * kInvTwoPi);
+        B.A2f = (float)A2;
+        B.e2f = (float)e2;
+        double vr = varpi - 2.0 * kPi * floor(varpi * kInvTwoPi);
         B.varpif = (float)vr;
-        B.sinvarpif = (float)sin(B.varpi);
+        B.sinvarpif = (float)sin(varpi);
     }
     B.di = B.ni = B.gi = 0;
     B.eS = B.eD = 0;
@@ -1356,61 +1329,128 @@ __device__ __forceinline__ void fft_dif_d(double2 *buf, int nsub, int lg)
 // ----------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------
+// One Newton iteration after another on Kepler's equation from u (FP64), for
+// the third-body pre-pass where its series does not apply (periods of days,
+// eccentricities close to 1); at most 20.
+__device__ __noinline__ double kepler_newton(double u, double l, double e, const double2 *__restrict__ sct)
+{
+    for (int it = 0; it < 20; it++) {
+        double s, c;
+        sincos_tab(u, sct, s, c);
+        const double f = fma(-e, s, u) - l, f1 = fma(-e, c, 1.0);
+        const double d = f / (f1 - 0.5 * f * (e * s) / f1);
+        u -= d;
+        if (!(fabs(d) > 1e-7)) break;
+    }
+    return u;
+}
+
+// v_LOS of the three spacecraft at one sample (gbgpu/thirdbody.py:228-380), at
+// the delayed times x0, x0 - del1, x0 - del2.  The eccentric anomaly u0 of
+// spacecraft 1 comes from the FP32 solve; with g = (u0 - e sin u0 - l)/(1 - e cos u0)
+// ~ 1e-6 for every spacecraft (their mean anomalies differ by n2 del, del < 9 s)
+// the exact anomalies are u0 + d, d the reversion of the Taylor series at u0 to
+// g^3 (the terms beyond the first in FP32), so one FP64 sincos and one
+// reciprocal serve all three, and sin, cos and 1/(1 - e cos) at u0 + d follow
+// from those at u0.  x0l is what the rounding of x0 left off; it and the rounding
+// of n2 (x0 - T2) go into l.  A swap step of 1,024 pairs of N = 512 (1,971 FP64
+// instructions per sample with a starter, a Newton step, two sincos, sin and
+// atan2 per spacecraft, now 580): 3.64 -> 1.41 ms.
+__device__ __forceinline__ void vlos3_fp64(const Bin &B, double x0, double x0l, double del1, double del2,
+                                           const double2 *__restrict__ sct, double v[3])
+{
+    constexpr double kRound = 6755399441055744.0;
+    const double e = B.kep.e2, eD = B.kep.eD;
+    const double dx = x0 - B.T2, M = B.n2 * dx;
+    const double k = fma(M, kInvTwoPi, kRound) - kRound;
+    const double l = fma(-k, kTwoPi, M) + fma(-k, kTwoPiLo, fma(B.n2, x0l, fma(B.n2, dx, -M)));
+    const float lf = d2f_scaled(l, 0);
+    const float uf = kepler_solve_f(fminf(fabsf(lf), (float)kPi), B.e2f);
+    const double u0 = f2d_bits(lf < 0.0f ? -uf : uf);
+    double su, cu;
+    sincos_tab(u0, sct, su, cu);
+    const double f1 = fma(-e, cu, 1.0), i1 = recip_fp64(f1);
+    const double f = fma(-e, su, u0) - l;
+    const float suf = d2f_scaled(su, 0), cuf = d2f_scaled(cu, 0), i1f = d2f_scaled(i1, 0);
+    const float a = 0.5f * B.e2f * suf * i1f, b = (1.0f / 6.0f) * B.e2f * cuf * i1f;
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+        const double dm = B.n2 * (s == 1 ? del1 : del2);
+        const double g = (s == 0 ? f : f + dm) * i1;
+        const float gf = d2f_scaled(g, 0);
+        double sn, cs, i;
+        if (fabsf(gf) * fmaxf(1.0f, fabsf(a)) < 1e-5f) {
+            const double d = -(g + f2d_bits(gf * gf * fmaf(fmaf(2.0f * a, a, -b), gf, a)));
+            const float df = d2f_scaled(d, 0);
+            sn = fma(d, cu + f2d_bits(df * fmaf(df * (-1.0f / 6.0f), cuf, -0.5f * suf)), su);
+            cs = fma(d, f2d_bits(df * fmaf(df * (1.0f / 6.0f), suf, -0.5f * cuf)) - su, cu);
+            // 1/(1 - eD cos u) from 1/f1: x = 1 - (1 - eD cos u)/f1
+            const double x = fma(-fma(-eD, cs, 1.0), i1, 1.0);
+            const float xf = d2f_scaled(x, 0);
+            i = fma(i1, x + f2d_bits(xf * fmaf(xf, xf, xf)), i1);
+        } else {
+            const double u = kepler_newton(u0, s == 0 ? l : l - dm, e, sct);
+            sincos_tab(u, sct, sn, cs);
+            i = 1.0 / fma(-eD, cs, 1.0);
+        }
+        v[s] = fma(i, fma(B.kep.ka, sn, B.kep.kb * cs), B.kep.kc);
+    }
+}
+
 // Third-body pre-passes (gbgpu/thirdbody.py:155-226) for a tile of cnt
 // binaries with N = 2^lg samples:
-//   A) v_LOS at every (sample, spacecraft) -> vl, and g = v_LOS f_GW;
+//   A) k.P/c of every spacecraft -> kps, v_LOS -> vl, and g = v_LOS f_GW -> psi
+//      (f_GW without fddot del^2/2, < 1e-21 of it);
 //   B) trapezoid increments (xi_n - xi_{n-1}) (g_{n-1} + g_n) pi / c -> inc;
 //   C) their inclusive prefix sum along n -> psi (the phase added to argS).
-// FP64 throughout; inc is scratch of 3 cnt N doubles.
+// FP64 throughout; inc and kps are scratch of 3 cnt N doubles each.
 // Called by every thread of the block (contains barriers).
 __device__ __forceinline__ void third_prepass(const Bin *bins, const double *__restrict__ tab,
-                                              int cnt, int lg, double step, double *psi, double *vl,
-                                              double *inc)
+                                              int cnt, int lg, double step, double Loc,
+                                              const double2 *__restrict__ sct, double *psi,
+                                              double *vl, double *inc, double *kps)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int N = 1 << lg, S = cnt << lg;
     for (int m = tid; m < S; m += kBlock) {
         const int p = m >> lg, n = m & (N - 1);
         const Bin &B = bins[p];
-        const double tm = (double)n * step;
-        if (!B.valid) {                       // outputs unused: no Kepler solves
+        double v[3] = {0.0, 0.0, 0.0}, kP[3] = {0.0, 0.0, 0.0}, fg[3] = {0.0, 0.0, 0.0};
+        if (B.valid) {                        // else outputs unused: no Kepler solve
+            double kr[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-            for (int s = 0; s < 3; s++) {
-                psi[(p * 3 + s) * N + n] = 0.0;
-                vl[(p * 3 + s) * N + n] = 0.0;
+            for (int c = 0; c < 3; c++) {
+                kP[0] = fma(B.k[c], __ldg(tab + (size_t)c * N + n), kP[0]);
+                kr[0] = fma(B.k[c], __ldg(tab + (size_t)(9 + c) * N + n), kr[0]);
+                kr[1] = fma(B.k[c], __ldg(tab + (size_t)(12 + c) * N + n), kr[1]);
             }
-            continue;
+            const double tm = f2d_bits((float)n) * step, xi = tm - kP[0];
+            const double del1 = Loc * kr[0], del2 = Loc * (kr[0] + kr[1]);
+            kP[1] = kP[0] + del1;
+            kP[2] = kP[0] + del2;
+            vlos3_fp64(B, xi, (tm - xi) - kP[0], del1, del2, sct, v);
+            const double fd = fma(B.fddot, xi, B.fdot);
+            fg[0] = fma(xi, 0.5 * (fd + B.fdot), B.f0);
+            fg[1] = fma(-del1, fd, fg[0]);
+            fg[2] = fma(-del2, fd, fg[0]);
         }
 #pragma unroll
         for (int s = 0; s < 3; s++) {
-            double kP = B.k[0] * __ldg(tab + (size_t)(3 * s) * N + n) +
-                        B.k[1] * __ldg(tab + (size_t)(3 * s + 1) * N + n) +
-                        B.k[2] * __ldg(tab + (size_t)(3 * s + 2) * N + n);
-            double xi = tm - kP;
-            double v = vlos_fp64(xi, B);
-            double fgw = B.f0 + B.fdot * xi + 0.5 * B.fddot * xi * xi;
-            psi[(p * 3 + s) * N + n] = v * fgw;
-            vl[(p * 3 + s) * N + n] = v;
+            kps[(p * 3 + s) * N + n] = kP[s];
+            vl[(p * 3 + s) * N + n] = v[s];
+            psi[(p * 3 + s) * N + n] = v[s] * fg[s];
         }
     }
     __syncthreads();
     for (int m = tid; m < S; m += kBlock) {
         const int p = m >> lg, n = m & (N - 1);
-        const Bin &B = bins[p];
 #pragma unroll
         for (int s = 0; s < 3; s++) {
+            const int o = (p * 3 + s) * N + n;
             double v = 0.0;
-            if (n > 0) {
-                double d = step;
-#pragma unroll
-                for (int c = 0; c < 3; c++)
-                    d -= B.k[c] * (__ldg(tab + (size_t)(3 * s + c) * N + n) -
-                                   __ldg(tab + (size_t)(3 * s + c) * N + n - 1));
-                // xi_n - xi_{n-1} = step - (kP_n - kP_{n-1})
-                v = d * (psi[(p * 3 + s) * N + n - 1] + psi[(p * 3 + s) * N + n]) / 2.0 *
-                    kPi * 2.0 / kCSI;
-            }
-            inc[(p * 3 + s) * N + n] = v;
+            // xi_n - xi_{n-1} = step - (kP_n - kP_{n-1})
+            if (n > 0) v = (step - (kps[o] - kps[o - 1])) * (kPi / kCSI) * (psi[o - 1] + psi[o]);
+            inc[o] = v;
         }
     }
     __syncthreads();
@@ -1632,8 +1672,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
             if constexpr (sizeof(R) == 8) {
                 psi = reinterpret_cast<double *>(buf + 3 * (size_t)maxcnt * N);
                 vl = reinterpret_cast<R *>(psi + 3 * (size_t)maxcnt * N);
-                third_prepass(bins, tab, cnt, lg, step, psi, reinterpret_cast<double *>(vl),
-                              reinterpret_cast<double *>(buf));
+                double *scr = reinterpret_cast<double *>(buf);
+                third_prepass(bins, tab, cnt, lg, step, K.Loc, sct, psi, vl, scr,
+                              scr + 3 * (size_t)maxcnt * N);
             } else {
                 // scratch: k.P/c and g in buf (6 floats per sample there)
                 psif = reinterpret_cast<dfl *>(buf + 3 * (size_t)maxcnt * N);
