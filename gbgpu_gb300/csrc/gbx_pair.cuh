@@ -335,40 +335,27 @@ __device__ __forceinline__ void slow_pair_unequal(const dfl (&r)[3][3], const df
 }
 
 // ---------------------------------------------------------------- slow part
-// The slow part at one sample (gbgpu.py:399-540 and 348-375), as slow_mixed
-// but every quantity a pair.  AE: out[0], out[1] = A, E (formed before the
-// transform); otherwise out[0..2] = X, Y, Z.  Amplitude divided out.
-//
-// Each link carries its spacecraft's carrier in one exponential:
-//   G_q = sinc(a_q) exp(-i (a_q + phi_s)) A_arm / 4
-// (one sincos of the summed angle instead of exp(-i a_q) times
-// exp(-i phi_s)), and with X' = G21 - G31, D_1 = G12 - G13 (cyclic) the TDI
-// combination X = fc2 (X' + fc D_1) (gbgpu.py:370-375) gives
-//   A = fc2/sqrt2 [(Z' - X') + fc (D_3 - D_1)],
-//   E = fc2/sqrt6 [(X' - 2Y' + Z') + fc (D_1 - 2 D_2 + D_3)]:
-// four complex products for A and E.
-template <bool AE, bool UNEQ>
-__device__ __forceinline__ void slow_pair(const Bin &B, int n, int N, dfl step, dfl Loc,
-                                          const double *__restrict__ tab,
-                                          const float4 *__restrict__ sct, cpx out[3], int tdi)
+// The general path, used with unequal arms: every link with its own argument,
+// every spacecraft with its own carrier (gbgpu.py:399-540 and 348-375).
+template <bool AE>
+__device__ __forceinline__ void slow_pair_links(const Bin &B, int n, int N, dfl step, dfl Loc,
+                                                const double *__restrict__ tab,
+                                                const float4 *__restrict__ sct, cpx out[3], int tdi)
 {
     const float *tabf = reinterpret_cast<const float *>(tab + (size_t)18 * N);
-    // arm vectors r_12, r_23, r_31 = (P_j - P_i)/L close (sum to zero to
-    // ~1e-14): with equal arms, arm 3's projections are minus the sum of the
-    // other two; the unequal-arm model reads all three (it needs |r_a|)
-    constexpr int NA = UNEQ ? 3 : 2;
-    dfl r[3][3];
+    dfl r[3][3], kr[3];
+    cpx A[3];
 #pragma unroll
-    for (int a = 0; a < NA; a++)
+    for (int a = 0; a < 3; a++) {
 #pragma unroll
         for (int c = 0; c < 3; c++)
             r[a][c] = {__ldg(tabf + (size_t)(3 * a + c) * N + n),
                        __ldg(tabf + (size_t)(27 + 3 * a + c) * N + n)};
-    dfl kr[3];
-#pragma unroll
-    for (int a = 0; a < NA; a++)
         kr[a] = u_dot3(B.kd[0], r[a][0], B.kd[1], r[a][1], B.kd[2], r[a][2]);
-    if constexpr (!UNEQ) kr[2] = df_neg(u_add(kr[0], kr[1]));
+        const dfl ru = u_dot3(B.pr.up[0], r[a][0], B.pr.up[1], r[a][1], B.pr.up[2], r[a][2]);
+        const dfl rv = u_dot3(B.pr.vp[0], r[a][0], B.pr.vp[1], r[a][1], B.pr.vp[2], r[a][2]);
+        A[a] = {p_mul(B.pr.ap4, u_dot2(rv, rv, df_neg(ru), ru)), p_mul(B.pr.ci, p_mul(ru, rv))};
+    }
     const dfl tm = p_mulf(step, (float)n);                 // n T/N
     const float tf = tm.h;
     const dfl tm2 = p_sqr(tm);
@@ -390,107 +377,217 @@ __device__ __forceinline__ void slow_pair(const Bin &B, int n, int N, dfl step, 
     // fdot = 1e-15 that term is 1e-3 of w0, and omL enters fc2 squared
     const dfl base = u_addf(dfl{B.w0h, B.w0l}, p_mul(dfl{B.w1, B.w1l}, tm));
     cpx E[3];
-    dfl fo[3], phs[3];
+    dfl fo[3];
 #pragma unroll
     for (int s = 0; s < 3; s++) {
         dfl ph = s == 0 ? ph0 : p_add(ph0, p_mul(dk[s], wt));
         const float kPf = kP0.h + dk[s].h;
         ph.l += kPf * kPf * fmaf(kPf, B.p3d.h, -(float)kPi * fdt);   // below 1e-8 rad
-        phs[s] = ph;
-        if constexpr (UNEQ) {
-            dfl cs, sn;
-            sincos_pair(ph, sct, cs, sn);
-            E[s] = {cs, df_neg(sn)};
-        }
+        dfl cs, sn;
+        sincos_pair(ph, sct, cs, sn);
+        E[s] = {cs, df_neg(sn)};
         // f(xi)/fstar at xi = t - kP: - w1 kP + w2 xi^2 are below 3e-6 of w0
         const float xf = tf - kPf;
         fo[s] = u_addf(base, dfl{fmaf(B.w2 * xf, xf, -B.w1 * kPf), 0.f});
     }
-    // antenna patterns per arm, with the 1/4 of the transfer functions:
-    // r.e+.r = (r.v)^2 - (r.u)^2, r.ex.r = 2 (r.u)(r.v)
-    cpx A[3];
-    dfl rus[2], rvs[2];
+    slow_pair_unequal<AE>(r, kr, fo, E, A, p_addf(base, dfl{B.w2 * tf * tf, 0.f}), tdi, sct, out);
+}
+
+// sum p and difference m of sin(a)/a at a = h + al and h - al (|al| <= h).
+// With q+- = (h +- al)^2 = sig +- tau, sig = h^2 + al^2, tau = 2 h al, the
+// series' terms combine: with rho = sig^2 + tau^2
+//   p = 2 - sig/3 + rho/60 - sig (rho + 2 tau^2)/2520 + ...
+//   m = tau [-1/3 + sig/30 - (rho + 2 sig^2)/2520 + ...],
+// the first three terms of each in pairs and the rest in FP32 at q+ and q-,
+// which rounds at most 1.5e-12 while q+ < 0.4; above that the fourth term is a
+// pair too (windows of 12-25 mHz within 2.5e-12 of long double; 2.1e-11 without
+// it, 1.4e-11 with the third and fourth terms' sum in FP32 over q^2).  From
+// |a| = 1.6 on the two sinc_pair themselves.  h2 = h^2.
+__device__ __forceinline__ void sinc_sum_pair(dfl h, dfl h2, dfl al, const float4 *__restrict__ tab,
+                                              dfl &p, dfl &m)
+{
+    if (h.h + fabsf(al.h) < 1.6f) {
+        const dfl sig = u_addf(h2, p_sqr(al));
+        const dfl tau = p_mul(p_scale(h, 2.f), al);
+        const dfl tau2 = p_sqr(tau), sig2 = p_sqr(sig);
+        const dfl rho = u_addf(sig2, tau2);
+        const float xp = sig.h + tau.h, xm = sig.h - tau.h;
+        // (df_fast where an FP32 tail enters: it reaches 1e-3 of the head, too
+        // much for a pair's tail)
+        dfl b = p_mul(dconst(1.0 / 60.0), rho);
+        dfl c = p_mul(dconst(1.0 / 30.0), sig);
+        float tp, tm;
+        if (fmaxf(xp, xm) < 0.4f) {
+            auto tail = [](float x) {
+                float q = fmaf(x, 1.0f / 6227020800.0f, -1.0f / 39916800.0f);
+                q = fmaf(q, x, 1.0f / 362880.0f);
+                return x * x * x * fmaf(q, x, -1.0f / 5040.0f);
+            };
+            tp = tail(xp);
+            tm = tail(xm);
+        } else {
+            auto tail = [](float x) {
+                float q = fmaf(x, 1.0f / 355687428096000.0f, -1.0f / 1307674368000.0f);
+                q = fmaf(q, x, 1.0f / 6227020800.0f);
+                q = fmaf(q, x, -1.0f / 39916800.0f);
+                q = fmaf(q, x, 1.0f / 362880.0f);
+                const float x2 = x * x;
+                return x2 * x2 * q;
+            };
+            tp = tail(xp);
+            tm = tail(xm);
+            const dfl k = dconst(-1.0 / 2520.0);
+            b = u_addf(b, p_mul(k, p_mul(sig, u_addf(rho, p_scale(tau2, 2.f)))));
+            c = u_addf(c, p_mul(k, u_addf(rho, p_scale(sig2, 2.f))));
+        }
+        p = u_addf(dfl{2.f, 0.f}, u_addf(p_mul(dconst(-1.0 / 3.0), sig), df_fast(b.h, b.l + (tp + tm))));
+        const dfl t = p_mul(tau, u_addf(dconst(-1.0 / 3.0), c));
+        m = df_fast(t.h, t.l + (tp - tm));
+    } else {
+        const dfl Sp = sinc_pair(u_add(h, al), tab), Sm = sinc_pair(u_sub(h, al), tab);
+        p = u_add(Sp, Sm);
+        m = u_sub(Sp, Sm);
+    }
+}
+
+// Equal arms: out[0], out[1] = A, E (AE, formed before the transform) or
+// out[0..2] = X, Y, Z at one sample, amplitude divided out.  The same
+// combination as slow_fp64 (gbx_wave.cu), every quantity a pair: with
+// h = omL/2, c, s = cos h, sin h, p, m = the sum and difference of the two
+// links' sin(a)/a and z_a = A_a exp(-i (th_a + 3h)),
+//   U = (p c + i m c d/2) z, V = (m s + i p s d/2) z,
+//   A = g4/sqrt2 [2 U_3 - U_1 - U_2 + i (V_1 - V_2)],
+//   E = g4/sqrt6 [3 (U_1 - U_2) + i (V_1 + V_2 - 2 V_3)], g4 = 4 omL sin omL:
+// one sincos, one joint sinc series and two real-by-complex products per arm,
+// and no complex product for the TDI factors.
+//
+// Angles: the links' arguments are a+- = h' (1 +- k.r) with h' = h - dl/2, dl
+// = f(t)/f* - f(xi_1)/f*, so with al_a = h' k.r_a
+//   th_1 + 3h = Th + al_1, th_2 + 3h = Th + al_1 + (al_1 + al_2),
+//   th_3 + 3h = Th + (al_1 + al_2), Th = phase_1 + 4h,
+// and what is left of the delays (k.P^2 terms, dl, d = -(L/c)^2 pi fd k.r, all
+// below 1e-8 rad) goes into the tails in FP32.
+//
+// Bound: FP32 pipe and its register ports.  An FMA with three different
+// registers takes two cycles (0.50 per cycle and scheduler measured, additions
+// 0.9; packed f32x2 operations have the same rates per value), so a pair
+// product costs 7 cycles and a sum 8.8, and fewer of both is what helps: 948 M
+// warp instructions for 20,000 binaries of uneven N against 1,069 M with two
+// sinc series, a complex product and the TDI factors' complex products per
+// link (200,000 binaries, default tiles: 12.36 -> 11.03 ms).
+template <bool AE>
+__device__ __forceinline__ void slow_pair(const Bin &B, int n, int N, dfl step, dfl Loc,
+                                          const double *__restrict__ tab,
+                                          const float4 *__restrict__ sct, cpx out[3])
+{
+    const float *tabf = reinterpret_cast<const float *>(tab + (size_t)18 * N);
+    // arm vectors r_12, r_23, r_31 = (P_j - P_i)/L close (sum to zero to
+    // ~1e-14): arm 3's projections are minus the sum of the other two
+    dfl kr[2], ru[3], rv[3];
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        dfl r[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            r[c] = {__ldg(tabf + (size_t)(3 * a + c) * N + n),
+                    __ldg(tabf + (size_t)(27 + 3 * a + c) * N + n)};
+        kr[a] = u_dot3(B.kd[0], r[0], B.kd[1], r[1], B.kd[2], r[2]);
+        ru[a] = u_dot3(B.pr.up[0], r[0], B.pr.up[1], r[1], B.pr.up[2], r[2]);
+        rv[a] = u_dot3(B.pr.vp[0], r[0], B.pr.vp[1], r[1], B.pr.vp[2], r[2]);
+    }
+    // (arm 3 enters by ru^2, rv^2 and ru rv: the sign does not matter)
+    ru[2] = u_add(ru[0], ru[1]);
+    rv[2] = u_add(rv[0], rv[1]);
+    const dfl tm = p_mulf(step, (float)n);                 // n T/N
+    const float tf = tm.h;
+    // carrier phase of spacecraft 1 (the expansion in slow_mixed):
+    //   -Phi0(tm) + kP w(tm) - pi kP^2 fd(tm) + pi/3 fddot kP^3
+    const dfl Phi0 = p_add(p_mul(u_add(B.omdfad, p_mul(u_add(B.pfd, p_mul(B.p3d, tm)), tm)), tm), B.phi0d);
+    const dfl wt = u_add(B.omd, p_mul(u_add(B.tpfd, p_mul(B.pfddd, tm)), tm));
+    const dfl kP0 = kP1_pair(B, tabf, N, n);
+    const dfl h = p_scale(p_mul(wt, Loc), 0.5f);           // omL/2
+    dfl Th = p_add(p_add(p_mul(kP0, wt), df_neg(Phi0)), p_scale(h, 4.f));
+    {
+        const float q = rintf(Th.h * (float)kInvTwoPi);
+        Th = p_add(Th, df_neg(p_mulf(dconst(kTwoPi), q)));
+    }
+    // FP32 terms per arm: sml_s = the k.P^2 and k.P^3 terms of spacecraft s's
+    // phase, K = 2 pi (L/c)^2 fd, d/2 = -K k.r/4
+    const float fdt = fmaf(B.fddotf, tf, B.fdotf);
+    const float kP = kP0.h;
+    const float dl = kP * fmaf(B.w2, tf + tf - kP, B.w1);
+    const float Kf = (float)kTwoPi * Loc.h * Loc.h * fdt;
+    const float kr2 = -(kr[0].h + kr[1].h);
+    const float krf[3] = {kr[0].h, kr[1].h, kr2};
+    float d2[3], tl[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        dfl ru, rv;
-        if (a < NA) {
-            ru = u_dot3(B.pr.ud[0], r[a][0], B.pr.ud[1], r[a][1], B.pr.ud[2], r[a][2]);
-            rv = u_dot2(B.pr.vd[0], r[a][0], B.pr.vd[1], r[a][1]);
-        } else {
-            ru = df_neg(u_add(rus[0], rus[1]));
-            rv = df_neg(u_add(rvs[0], rvs[1]));
-        }
-        if (a < 2) {
-            rus[a] = ru;
-            rvs[a] = rv;
-        }
-        const dfl pp = p_scale(u_dot2(rv, rv, df_neg(ru), ru), 0.25f);
-        const dfl cc = p_scale(p_mul(ru, rv), 0.5f);
-        A[a] = {u_dot2(pp, B.pr.DP.x, cc, B.pr.DC.x), u_dot2(pp, B.pr.DP.y, cc, B.pr.DC.y)};
+        d2[a] = -0.25f * Kf * krf[a];
+        const float kk = a == 0 ? 0.f : a == 1 ? krf[0] : -kr2;         // del_a / (L/c)
+        const float kPa = fmaf(Loc.h, kk, kP);
+        tl[a] = kPa * kPa * fmaf(kPa, B.p3d.h, -(float)kPi * fdt) + fmaf(kk, dl, -0.5f * dl) +
+                (d2[a] - 0.5f * Kf * kk * (1.f + krf[a]));
     }
-    if constexpr (UNEQ) {
-        slow_pair_unequal<AE>(r, kr, fo, E, A, p_addf(base, dfl{B.w2 * tf * tf, 0.f}), tdi, sct, out);
-        return;
+    dfl hp = h;
+    hp.l = fmaf(-0.5f, dl, hp.l);
+    const dfl h2 = p_sqr(hp);
+    dfl al[3], th[3];
+    al[0] = p_mul(kr[0], hp);
+    al[1] = p_mul(kr[1], hp);
+    const dfl a01 = u_add(al[0], al[1]);
+    al[2] = df_neg(a01);
+    th[0] = u_add(Th, al[0]);
+    th[1] = u_add(th[0], a01);
+    th[2] = u_add(Th, a01);
+    // cos h, and sin h to relative accuracy (it scales the window through g4)
+    dfl c, s;
+    if (h.h < 0.16f) {
+        dfl S;
+        sinc_cos_pair(h, sct, S, c);
+        s = p_mul(h, S);
+    } else {
+        sincos_pair_acc(h, sct, c, s);
     }
-    // links (ij, arm, spacecraft): 12,23,31 (+k.r) and 21,32,13 (-k.r); the two
-    // links of arm a (spacecraft a and a+1) carry angles th+ = a+ + phi_a and
-    // th- = a- + phi_(a+1) that differ by
-    //   d = (fo_(a+1) - fo_a)/2 + k.r (f(t)/f* - (fo_a + fo_(a+1))/2) + (k.P^2 terms),
-    // |d| < 1e-7 rad (fdot k.P/f* and the phase's k.P^2 terms), so
-    // exp(-i th-) A_a = exp(-i th+) A_a (1 - i d) to 1e-14: one pair sincos
-    // and one complex product per arm.  (|d| >= 1e-4 would take the full
-    // sincos; it does not occur for equal arms.)
-    cpx G[6];
+    cpx U[3], V[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const int s2 = a == 2 ? 0 : a + 1;
-        const dfl ap = p_scale(p_mul(fo[a], p_addf(dfl{1.f, 0.f}, kr[a])), 0.5f);
-        const dfl am = p_scale(p_mul(fo[s2], p_addf(dfl{1.f, 0.f}, df_neg(kr[a]))), 0.5f);
-        const dfl Sp = sinc_pair(ap, sct), Sm = sinc_pair(am, sct);
-        const dfl thp = u_add(ap, phs[a]), thm = u_add(am, phs[s2]);
-        dfl c, sn;
-        sincos_pair(thp, sct, c, sn);
-        const cpx eA = cu_mul(cpx{c, df_neg(sn)}, A[a]);
-        G[a] = {p_mul(Sp, eA.x), p_mul(Sp, eA.y)};
-        const dfl dl = u_sub(thm, thp);
-        const float d = dl.h + dl.l;
-        cpx eAm;
-        if (fabsf(d) < 1e-4f) {
-            eAm = {u_add(eA.x, dfl{d * eA.y.h, 0.f}), u_add(eA.y, dfl{-d * eA.x.h, 0.f})};
-        } else {
-            sincos_pair(thm, sct, c, sn);
-            eAm = cu_mul(cpx{c, df_neg(sn)}, A[a]);
-        }
-        G[a + 3] = {p_mul(Sm, eAm.x), p_mul(Sm, eAm.y)};
+        dfl p, m;
+        sinc_sum_pair(hp, h2, al[a], sct, p, m);
+        // antenna pattern r.e.r of the rotated basis, with the 1/4 of the
+        // transfer functions
+        const cpx A = {p_mul(B.pr.ap4, u_dot2(rv[a], rv[a], df_neg(ru[a]), ru[a])),
+                       p_mul(B.pr.ci, p_mul(ru[a], rv[a]))};
+        th[a].l += tl[a];
+        dfl cs, sn;
+        sincos_pair(th[a], sct, cs, sn);
+        const cpx z = cu_mul(cpx{cs, df_neg(sn)}, A);
+        const dfl P = p_mul(p, c), M = p_mul(m, s);
+        const float e1 = p.h * s.h * d2[a], e2 = m.h * c.h * d2[a];
+        U[a] = {p_mul(P, z.x), p_mul(P, z.y)};
+        U[a].x.l = fmaf(-e2, z.y.h, U[a].x.l);
+        U[a].y.l = fmaf(e2, z.x.h, U[a].y.l);
+        V[a] = {p_mul(M, z.x), p_mul(M, z.y)};
+        V[a].x.l = fmaf(-e1, z.y.h, V[a].x.l);
+        V[a].y.l = fmaf(e1, z.x.h, V[a].y.l);
     }
-    // omega L, fc = e^{-i omL}, fc2 = 4 omL sin(omL) fc (gbgpu.py:362-368)
-    const dfl omL = u_addf(base, dfl{B.w2 * tf * tf, 0.f});
-    dfl co, so;
-    sincos_pair_acc(omL, sct, co, so);   // sin(omL) scales the window: relative accuracy at low f
-    const cpx fc = {co, df_neg(so)};
-    const dfl g4 = p_scale(p_mul(omL, so), 4.f);
+    const dfl g4 = p_scale(p_mul(h, p_mul(s, c)), 16.f);    // 4 omL sin(omL)
     if constexpr (AE) {
-        // A = (Z - X)/sqrt2, E = (X - 2Y + Z)/sqrt6 (utility.py:24-38), with
-        //   Z' - X' = (G31 + G13) - (G23 + G21),  D3 - D1 = (G31 + G13) - (G12 + G32),
-        //   X' - 2Y' + Z' = 2 (G12 - G32) + (G21 - G23) + (G13 - G31),
-        //   D1 - 2 D2 + D3 = (G12 - G32) + 2 (G21 - G23) - (G13 - G31)
-        const cpx s25 = cu_add(G[2], G[5]);
-        const cpx ga = cu_sub(G[0], G[4]), gb = cu_sub(G[3], G[1]), gc = cu_sub(G[5], G[2]);
-        const cpx wA = cu_add(cu_sub(s25, cu_add(G[1], G[3])),
-                              cu_mul(fc, cu_sub(s25, cu_add(G[0], G[4]))));
-        const cpx wE = cu_add(cu_add(cp_pow2(ga, 2.f), cu_add(gb, gc)),
-                              cu_mul(fc, cu_sub(cu_add(ga, cp_pow2(gb, 2.f)), gc)));
+        // A = (Z - X)/sqrt2, E = (X - 2Y + Z)/sqrt6 (utility.py:24-38)
+        const cpx us = cu_add(U[0], U[1]), ud = cu_sub(U[0], U[1]);
+        const cpx vs = cu_add(V[0], V[1]), vd = cu_sub(V[0], V[1]);
+        const cpx tA = cu_sub(cp_pow2(U[2], 2.f), us), tE = cu_sub(vs, cp_pow2(V[2], 2.f));
         const dfl gA = p_mul(g4, dconst(0.70710678118654752440));
         const dfl gE = p_mul(g4, dconst(0.40824829046386301637));
-        out[0] = cu_mul(cpx{p_mul(gA, co), df_neg(p_mul(gA, so))}, wA);
-        out[1] = cu_mul(cpx{p_mul(gE, co), df_neg(p_mul(gE, so))}, wE);
+        out[0] = {p_mul(gA, u_sub(tA.x, vd.y)), p_mul(gA, u_add(tA.y, vd.x))};
+        out[1] = {p_mul(gE, u_sub(p_mulf(ud.x, 3.f), tE.y)), p_mul(gE, u_add(p_mulf(ud.y, 3.f), tE.x))};
     } else {
-        const cpx D1 = cu_sub(G[0], G[5]), D2 = cu_sub(G[1], G[3]), D3 = cu_sub(G[2], G[4]);
-        const cpx X0 = cu_sub(G[3], G[2]), Y0 = cu_sub(G[4], G[0]), Z0 = cu_sub(G[5], G[1]);
-        const cpx fc2 = {p_mul(g4, co), df_neg(p_mul(g4, so))};
-        out[0] = cu_mul(fc2, cu_add(X0, cu_mul(fc, D1)));
-        out[1] = cu_mul(fc2, cu_add(Y0, cu_mul(fc, D2)));
-        out[2] = cu_mul(fc2, cu_add(Z0, cu_mul(fc, D3)));
+        // X = g4 [(U_1 - i V_1) - (U_3 + i V_3)] and cyclic
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int e = q == 0 ? 2 : q - 1;
+            const cpx ud = cu_sub(U[q], U[e]), vs = cu_add(V[q], V[e]);
+            out[q] = {p_mul(g4, u_add(ud.x, vs.y)), p_mul(g4, u_sub(ud.y, vs.x))};
+        }
     }
 }
 
@@ -684,7 +781,8 @@ __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
             if (!B.valid) {
                 o[0] = o[1] = o[2] = cp_zero();
             } else {
-                slow_pair<NCH == 2, UNEQ>(B, n, N, stepd, K.Locd, tab, sct, o, a.tdi2);
+                if constexpr (UNEQ) slow_pair_links<NCH == 2>(B, n, N, stepd, K.Locd, tab, sct, o, a.tdi2);
+                else slow_pair<NCH == 2>(B, n, N, stepd, K.Locd, tab, sct, o);
             }
 #pragma unroll
             for (int c = 0; c < NCH; c++) buf[(p * NCH + c) * N + swz(n, lg)] = o[c];

@@ -65,8 +65,8 @@ struct __align__(16) Bin {
             double pf2, p3f3;      // 2 pi fdot, pi fddot
         } q;
         struct {
-            dfl ud[3], vd[2];      // u and v (v has no z component) as pairs (pair form)
-            cpx DP, DC;            // polarisation factors divided by amp, as pairs
+            dfl up[3], vp[3];      // the same as pairs (pair form)
+            dfl ap4, ci;
         } pr;
     };
     double2 DP, DC;                // polarisation factors divided by amp
@@ -443,18 +443,25 @@ __device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     double u[3] = {ct * cp, ct * sp, -st};
     double v[3] = {sp, -cp, 0.0};
     B.k[0] = -st * cp; B.k[1] = -st * sp; B.k[2] = -ct;
+    // r.e+.r DP + r.ex.r DC = (r.v + i r.u)^2 with its real part times
+    // 1 + cos^2 iota and its imaginary part times 2 cos iota after a turn by
+    // 2 psi: the turn goes into the basis, v' + i u' = (v + i u) e^{i psi}
+    double vp[3], up[3];
+    for (int c = 0; c < 3; c++) {
+        vp[c] = v[c] * c1p - u[c] * s1p;
+        up[c] = v[c] * s1p + u[c] * c1p;
+    }
     if (a.precision == GBX_PAIR) {
-        for (int c = 0; c < 3; c++) B.pr.ud[c] = df_from(u[c]);
-        for (int c = 0; c < 2; c++) B.pr.vd[c] = df_from(v[c]);
-        B.pr.DP = {df_from(B.DP.x), df_from(B.DP.y)};
-        B.pr.DC = {df_from(B.DC.x), df_from(B.DC.y)};
-    } else {
-        // r.e+.r DP + r.ex.r DC = (r.v + i r.u)^2 with its real part times
-        // 1 + cos^2 iota and its imaginary part times 2 cos iota after a turn by
-        // 2 psi: the turn goes into the basis, v' + i u' = (v + i u) e^{i psi}
         for (int c = 0; c < 3; c++) {
-            B.q.vp[c] = v[c] * c1p - u[c] * s1p;
-            B.q.up[c] = v[c] * s1p + u[c] * c1p;
+            B.pr.up[c] = df_from(up[c]);
+            B.pr.vp[c] = df_from(vp[c]);
+        }
+        B.pr.ap4 = df_from(0.25 * Ap);
+        B.pr.ci = df_from(ci);
+    } else if (a.precision == GBX_FP64) {
+        for (int c = 0; c < 3; c++) {
+            B.q.up[c] = up[c];
+            B.q.vp[c] = vp[c];
         }
         B.q.ap4 = 0.25 * Ap;
         B.q.ci = ci;
