@@ -702,10 +702,61 @@ __device__ __forceinline__ void fft_dif_pair(cpx *buf, int nsub, int lg)
     __syncthreads();
 }
 
+// ---------------------------------------------------------------- outputs
+// (h + l) 2^e as a double, |e| < 700, without an FP64 instruction: the bits of
+// h widened, and l added to them as a whole number of units in the last place
+// of the result (truncated; half that unit below a power of two).  Tails below
+// FP32's normal range count as zero.
+__device__ __forceinline__ double pair_to_double(dfl a, int e)
+{
+    a = df_fast(a.h, a.l);
+    const unsigned u = __float_as_uint(a.h), v = __float_as_uint(a.l);
+    const int eh = (u >> 23) & 0xffu, el = (v >> 23) & 0xffu;
+    const unsigned hi = (u & 0x80000000u) | ((unsigned)(eh + 896 + e) << 20) | ((u & 0x7fffffu) >> 3);
+    const unsigned ml = (v & 0x7fffffu) | 0x800000u;
+    const bool neg = (int)(u ^ v) < 0;
+    const int sh = el - eh + (neg && (u & 0x7fffffu) == 0 ? 30 : 29);
+    const unsigned k = el == 0 || sh <= -24 ? 0u : (sh >= 0 ? ml << sh : ml >> -sh);
+    unsigned long long w = ((unsigned long long)hi << 32) | (unsigned long long)(u << 29);
+    w = neg ? w - k : w + k;
+    if (eh == 0) w = (unsigned long long)(u & 0x80000000u) << 32;
+    if (eh == 0xff) w = (unsigned long long)((u & 0x80000000u) | 0x7ff00000u | ((u & 0x7fffffu) ? 0x80000u : 0u)) << 32;
+    return __longlong_as_double((long long)w);
+}
+
+// A binary's output scale as a pair times 2^e: the pair form's windows are
+// multiplied by it in pairs (their error is ~2e-12, the product's 1e-14) and
+// widened on the integer pipe, because one FP64 instruction takes the issue
+// time of 64 FP32 ones.  mode 0: exponent out of range (also zero, infinite or
+// NaN scales), products in FP64; 1: real; 2: complex (TDI-2).
+struct PairScale {
+    cpx m;
+    int e, mode;
+};
+
+__device__ __forceinline__ void set_pair_scale(PairScale &P, double2 sc)
+{
+    const int ex = max(__double2hiint(sc.x) & 0x7fffffff, __double2hiint(sc.y) & 0x7fffffff) >> 20;
+    P.e = ex - 1023;
+    P.mode = P.e < -600 || P.e > 600 ? 0 : sc.y == 0.0 ? 1 : 2;
+    const double p2 = P.mode ? exp2_int(-P.e) : 0.0;
+    P.m = {df_from(sc.x * p2), df_from(sc.y * p2)};
+}
+
+__device__ __forceinline__ cpx pair_scaled(cpx z, const PairScale &P)
+{
+    return P.mode == 1 ? cp_scale(z, P.m.x) : cu_mul(z, P.m);
+}
+
+__device__ __forceinline__ double2 pair_out(cpx z, int e)
+{
+    return make_double2(pair_to_double(z.x, e), pair_to_double(z.y, e));
+}
+
 // ---------------------------------------------------------------- kernel
 // One CTA per tile as wave_kernel; MODE_WAVE writes the reference's output
-// arrays (the transformed pairs rounded once to FP64, then the FP64 scale
-// and AET), MODE_LL folds the window into <d|h> and <h|h> (pairs).  Shared memory: the binaries' constants, the reduction
+// arrays (X, Y, Z and A, E, T scaled and combined in pairs, widened to FP64),
+// MODE_LL folds the window into <d|h> and <h|h> (pairs).  Shared memory: the binaries' constants, the reduction
 // scratch, the sin/cos table and the transform buffers.
 template <int MODE, bool UNEQ>
 __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
@@ -718,6 +769,7 @@ __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
                                              sizeof(double) * red_doubles(K.maxS));
     cpx *buf = reinterpret_cast<cpx *>(sct + kScN);
     __shared__ int s_tile;
+    __shared__ PairScale s_sc[MODE == MODE_WAVE || MODE == MODE_FILL ? kMaxPack : 1];
 
     const gbx_wave_args &a = K.a;
     const int tid = threadIdx.x;
@@ -772,6 +824,7 @@ __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
         }
         __syncthreads();
 
+        if ((MODE == MODE_WAVE || MODE == MODE_FILL) && tid < cnt) set_pair_scale(s_sc[tid], bins[tid].scale);
         const int S = cnt << lg;
         const dfl stepd = K.stepd[lg];
         for (int m = tid; m < S; m += kBlock) {
@@ -797,24 +850,43 @@ __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
                 const Bin &B = bins[p];
                 if (B.b < 0) continue;
                 const int pos = swz(bitrev((i + (N >> 1)) & (N - 1), lg), lg);   // fftshift
-                const cpx X = buf[(p * 3 + 0) * N + pos], Y = buf[(p * 3 + 1) * N + pos],
-                          Z = buf[(p * 3 + 2) * N + pos];
-                const double2 Xd = cmul(make_double2(pd(X.x), pd(X.y)), B.scale);
-                const double2 Yd = cmul(make_double2(pd(Y.x), pd(Y.y)), B.scale);
-                const double2 Zd = cmul(make_double2(pd(Z.x), pd(Z.y)), B.scale);
+                cpx X = buf[(p * 3 + 0) * N + pos], Y = buf[(p * 3 + 1) * N + pos],
+                    Z = buf[(p * 3 + 2) * N + pos];
                 const size_t o = (size_t)B.b * 3 * N + i;
-                if (K.XYZ) {
-                    K.XYZ[o] = Xd;
-                    K.XYZ[o + N] = Yd;
-                    K.XYZ[o + 2 * N] = Zd;
-                }
-                if (K.AET) {
-                    const double is2 = 0.70710678118654752440, is6 = 0.40824829046386301637;
-                    const double i3 = 0.57735026918962576451;
-                    K.AET[o] = make_double2((Zd.x - Xd.x) * is2, (Zd.y - Xd.y) * is2);
-                    K.AET[o + N] = make_double2((Xd.x - 2.0 * Yd.x + Zd.x) * is6,
-                                                (Xd.y - 2.0 * Yd.y + Zd.y) * is6);
-                    K.AET[o + 2 * N] = make_double2((Xd.x + Yd.x + Zd.x) * i3, (Xd.y + Yd.y + Zd.y) * i3);
+                const PairScale &sc = s_sc[p];
+                if (sc.mode) {
+                    X = pair_scaled(X, sc);
+                    Y = pair_scaled(Y, sc);
+                    Z = pair_scaled(Z, sc);
+                    if (K.XYZ) {
+                        K.XYZ[o] = pair_out(X, sc.e);
+                        K.XYZ[o + N] = pair_out(Y, sc.e);
+                        K.XYZ[o + 2 * N] = pair_out(Z, sc.e);
+                    }
+                    if (K.AET) {
+                        const cpx xz = cu_add(X, Z);
+                        K.AET[o] = pair_out(cp_scale(cu_sub(Z, X), dconst(0.70710678118654752440)), sc.e);
+                        K.AET[o + N] = pair_out(cp_scale(cu_sub(xz, cp_pow2(Y, 2.f)),
+                                                         dconst(0.40824829046386301637)), sc.e);
+                        K.AET[o + 2 * N] = pair_out(cp_scale(cu_add(xz, Y), dconst(0.57735026918962576451)), sc.e);
+                    }
+                } else {
+                    const double2 Xd = cmul(make_double2(pd(X.x), pd(X.y)), B.scale);
+                    const double2 Yd = cmul(make_double2(pd(Y.x), pd(Y.y)), B.scale);
+                    const double2 Zd = cmul(make_double2(pd(Z.x), pd(Z.y)), B.scale);
+                    if (K.XYZ) {
+                        K.XYZ[o] = Xd;
+                        K.XYZ[o + N] = Yd;
+                        K.XYZ[o + 2 * N] = Zd;
+                    }
+                    if (K.AET) {
+                        const double is2 = 0.70710678118654752440, is6 = 0.40824829046386301637;
+                        const double i3 = 0.57735026918962576451;
+                        K.AET[o] = make_double2((Zd.x - Xd.x) * is2, (Zd.y - Xd.y) * is2);
+                        K.AET[o + N] = make_double2((Xd.x - 2.0 * Yd.x + Zd.x) * is6,
+                                                    (Xd.y - 2.0 * Yd.y + Zd.y) * is6);
+                        K.AET[o + 2 * N] = make_double2((Xd.x + Yd.x + Zd.x) * i3, (Xd.y + Yd.y + Zd.y) * i3);
+                    }
                 }
                 if (i == 0 && K.start_out) K.start_out[B.b] = B.start;
             }
@@ -921,7 +993,7 @@ __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
         } else if constexpr (MODE == MODE_FILL) {
             // as wave_kernel's MODE_FILL: each run of same-group binaries with
             // ascending, overlapping windows is summed once per bin of its span;
-            // the pairs are rounded once to FP64 and scaled in FP64
+            // the windows are scaled in pairs, widened, and summed in FP64
             __shared__ int s_run[kMaxPack + 1], s_lo[kMaxPack], s_off[kMaxPack + 1];
             __shared__ int s_nruns;
             if (tid == 0) s_nruns = fill_runs(bins, cnt, N, s_run, s_lo, s_off);
@@ -941,8 +1013,15 @@ __global__ void __launch_bounds__(kBlock, 2) pair_kernel(const KParams K)
                     if (i < 0 || i >= N) continue;
                     const int pos = swz(bitrev((i + (N >> 1)) & (N - 1), lg), lg);
                     const cpx tA = buf[(p * 2 + 0) * N + pos], tE = buf[(p * 2 + 1) * N + pos];
-                    const double2 a2 = cmul(make_double2(pd(tA.x), pd(tA.y)), B.scale);
-                    const double2 e2 = cmul(make_double2(pd(tE.x), pd(tE.y)), B.scale);
+                    const PairScale &sc = s_sc[p];
+                    double2 a2, e2;
+                    if (sc.mode) {
+                        a2 = pair_out(pair_scaled(tA, sc), sc.e);
+                        e2 = pair_out(pair_scaled(tE, sc), sc.e);
+                    } else {
+                        a2 = cmul(make_double2(pd(tA.x), pd(tA.y)), B.scale);
+                        e2 = cmul(make_double2(pd(tE.x), pd(tE.y)), B.scale);
+                    }
                     if (any) {
                         Ah = cadd(Ah, a2);
                         Eh = cadd(Eh, e2);
