@@ -602,9 +602,19 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
         const int i0 = tid - pq * Tpb;
         const int nproc = SWAP ? cnt >> 1 : cnt;
         const bool valid = p < cnt && bins[p].valid && (!SWAP || bins[p - 1].valid);
+        // FP32 sums over the bins or samples v, v + Tv, ... of a column v (Tv: the
+        // threads a binary has in a tile of kTileMin samples) and float pairs over
+        // the columns, as the likelihood: the result does not depend on the tile.
+        // (The third body's second pass goes on with the first one's FP32 sums,
+        // so a thread has one column there and the caller keeps the default tile.)
+        const int Tv = THIRD ? Tpb : (SWAP ? 2 : 1) * (kBlock / tile_pack(0, lg, SWAP ? 2 : 1));
         float acc[kGradAcc];
+        dfl tot[kGradAcc];
 #pragma unroll
-        for (int k = 0; k < kGradAcc; k++) acc[k] = 0.0f;
+        for (int k = 0; k < kGradAcc; k++) {
+            acc[k] = 0.0f;
+            tot[k] = dfl{0.f, 0.f};
+        }
         if (p < cnt) {
             const Bin &B = bins[p];
             bool out = false;
@@ -613,7 +623,8 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
             // SWAP: the current source's scale in the same units
             const Bin &Bo = bins[SWAP ? p - 1 : p];
             const float2 so = make_float2(d2f_scaled(Bo.scale.x, B.eD), d2f_scaled(Bo.scale.y, B.eD));
-            for (int i = i0; i < N; i += Tpb) {
+          for (int v = i0; v < Tv; v += Tpb) {
+            for (int i = v; i < N; i += Tv) {
                 const int j = B.start + i;
                 const int pos = bitrev((i + (N >> 1)) & (N - 1), lg);
                 const int sp = swz(pos, lg);
@@ -664,6 +675,14 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
                 buf[(p * 2 + 0) * N + sp] = make_float2(uA.x, -uA.y);
                 buf[(p * 2 + 1) * N + sp] = make_float2(uE.x, -uE.y);
             }
+            if (!THIRD) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    tot[k] = df_add(tot[k], dfl{acc[k], 0.f});
+                    acc[k] = 0.f;
+                }
+            }
+          }
             if (out) flag(a.status, GBX_FLAG_WINDOW);
         }
         __syncthreads();
@@ -674,7 +693,8 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
             const Bin &B = bins[p];
             const GradExtra &Gx = gxs[p];
             if (valid) {
-                for (int n = i0; n < N; n += Tpb) {
+              for (int v = i0; v < Tv; v += Tpb) {
+                for (int n = v; n < N; n += Tv) {
                     float2 Yc[3], Es[3];
                     float2 *ep = es + 3 * ((size_t)(p << lg) + n);
                     // Y_X, Y_Y, Y_Z from the transformed A, E weights
@@ -702,6 +722,14 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
                         slow_grad_mixed<false>(B, Gx, n, N, stepd, tab, ifs, fstarf, Yc, Es, acc + 5);
                     }
                 }
+                if (!THIRD) {
+#pragma unroll
+                    for (int k = 5; k < kGradAcc; k++) {
+                        tot[k] = df_add(tot[k], dfl{acc[k], 0.f});
+                        acc[k] = 0.f;
+                    }
+                }
+              }
             }
         }
         if (THIRD) {
@@ -753,7 +781,7 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
             const int g = tid / width;
 #pragma unroll
             for (int k = 0; k < kGradAcc; k++) {
-                dfl x = {acc[k], 0.f};
+                dfl x = THIRD ? dfl{acc[k], 0.f} : tot[k];
                 for (int o = width >> 1; o > 0; o >>= 1) {
                     dfl y = {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
                     x = df_add(x, y);

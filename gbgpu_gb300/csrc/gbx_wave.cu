@@ -1797,12 +1797,19 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
             const int i0 = tid - pr * Tp2;
             typedef typename std::conditional<sizeof(R) == 8, double, float>::type Acc;
             Acc acc8[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // Crn (2), Cro (2), Hn, Ho, Cx (2)
+            // mixed form: FP32 sums over columns of the default tile's threads,
+            // float pairs over the columns (as the likelihood)
+            dfl tot8[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) tot8[k] = dfl{0.f, 0.f};
+            const int Tv = sizeof(R) == 8 ? Tp2 : 2 * (kBlock / tile_pack(0, lg, 2));
             if (2 * pr + 1 < cnt) {
                 const Bin &Bo = bins[2 * pr], &Bn = bins[2 * pr + 1];
                 const int po = 2 * pr, pn = 2 * pr + 1;
                 if (Bo.valid && Bn.valid) {
                     bool out = false;
-                    for (int e = i0; e < 2 * N; e += Tp2) {
+                  for (int v = i0; v < Tv; v += Tp2) {
+                    for (int e = v; e < 2 * N; e += Tv) {
                         const bool isnew = e < N;
                         const int i = isnew ? e : e - N;
                         const Bin &Bw = isnew ? Bn : Bo;
@@ -1849,6 +1856,14 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                             acc8[2] += cr; acc8[3] += ci; acc8[5] += hh2;
                         }
                     }
+                    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            tot8[k] = df_add(tot8[k], dfl{acc8[k], 0.f});
+                            acc8[k] = 0;
+                        }
+                    }
+                  }
                     if (out) flag(a.status, GBX_FLAG_WINDOW);
                 }
             }
@@ -1863,7 +1878,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                         for (int o = width >> 1; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
                         if (leader) red[8 * g + k] = x;
                     } else {
-                        dfl x = {acc8[k], 0.f};
+                        dfl x = tot8[k];
                         for (int o = width >> 1; o > 0; o >>= 1) {
                             dfl y = {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
                             x = df_add(x, y);
@@ -1953,16 +1968,21 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
         } else {  // MODE_LL
             // Threads [p*Tpb, (p+1)*Tpb) own binary p of the tile and walk its
             // window with stride Tpb, so each warp reads a contiguous run of the
-            // data/PSD window.  Per-thread sums are FP64 (plain form) or FP32
-            // (mixed form; N/Tpb <= 16 terms), lanes are combined with an FP64 or
-            // float-pair shuffle tree, and a binary's <= 16 group partials are
-            // added by one thread per (binary, term).
+            // data/PSD window.  Sums are FP64 (plain form) or, in the mixed form,
+            // FP32 over the bins v, v + Tv, v + 2 Tv ... of a column v, Tv being
+            // the threads a binary has in a tile of kTileMin samples, and in
+            // float pairs over the columns: the FP32 sums (2 to 8 terms), and
+            // so the result, do not depend on the tile.  Lanes are combined with
+            // an FP64 or float-pair shuffle tree, and a binary's <= 16 group
+            // partials are added by one thread per (binary, term).
             const int Tpb = kBlock / maxcnt;               // 256 / binaries per tile
             const int width = Tpb < 32 ? Tpb : 32;
             const int p = tid / Tpb;
             const int i0 = tid - p * Tpb;
             typedef typename std::conditional<sizeof(R) == 8, double, float>::type Acc;
             Acc sr = 0, si = 0, sh = 0;
+            dfl xr = {0.f, 0.f}, xi = {0.f, 0.f}, xh = {0.f, 0.f};
+            const int Tv = sizeof(R) == 8 ? Tpb : kBlock / tile_pack(0, lg, 1);
             // one PSD array for both channels (the usual call): the channels'
             // terms are summed, then weighted once
             const bool samepsd = K.A_psd == K.E_psd;
@@ -1970,7 +1990,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                 const Bin &B = bins[p];
                 bool out = false;
                 if (B.valid) {
-                    for (int i = i0; i < N; i += Tpb) {
+                  for (int v = i0; v < Tv; v += Tpb) {
+                    for (int i = v; i < N; i += Tv) {
                         const int j = B.start + i;
                         if (j < 0 || j >= K.L) {
                             out = true;
@@ -2015,6 +2036,13 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                             sh += fmaf(hA.x, hA.x, hA.y * hA.y) * wA + fmaf(hE.x, hE.x, hE.y * hE.y) * wE;
                         }
                     }
+                    if constexpr (sizeof(R) == 4) {
+                        xr = df_add(xr, dfl{sr, 0.f});
+                        xi = df_add(xi, dfl{si, 0.f});
+                        xh = df_add(xh, dfl{sh, 0.f});
+                        sr = si = sh = 0;
+                    }
+                  }
                 }
                 if (out) flag(a.status, GBX_FLAG_WINDOW);
             }
@@ -2028,7 +2056,6 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                 }
                 gr = sr; gi = si; gh = sh;
             } else {
-                dfl xr = {sr, 0.f}, xi = {si, 0.f}, xh = {sh, 0.f};
                 for (int o = width >> 1; o > 0; o >>= 1) {
                     dfl yr = {__shfl_xor_sync(0xffffffffu, xr.h, o), __shfl_xor_sync(0xffffffffu, xr.l, o)};
                     dfl yi = {__shfl_xor_sync(0xffffffffu, xi.h, o), __shfl_xor_sync(0xffffffffu, xi.l, o)};

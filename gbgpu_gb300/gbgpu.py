@@ -121,6 +121,51 @@ def plan_tiles(N_per_bin, tile=0):
     return order, tiles
 
 
+def default_tile(kind, precision, nparams, counts, sms):
+    """Samples per tile when the autotuner is off, from the sizes alone.
+
+    A large tile packs more binaries into a block, whose fixed work (barriers,
+    constants, reductions, the queue) is then shared; ``counts`` lists
+    (N, binaries).  Upper end: the largest tile whose buffers leave an SM as
+    many blocks as the registers do (three for the mixed form's likelihood,
+    fill, swap and waveform kernels, two otherwise; bytes per sample below).
+    On one GB300, against 512 samples (us): gradient 8,191 x 512 691 -> 506,
+    mixed likelihood 50,000 x 256 660 -> 518, pair 1,314 -> 1,134, pair fill
+    60,000 x 512 3,466 -> 3,016; one step further costs 10-30 %.  The FP64 form
+    is bound by its FP64 instructions at any tile and stays at 512 (3,000 x
+    512: 1,079 at 512, 1,062 at 1024, 1,247 at 2048).  Lower end: a tile may
+    not leave the SMs without blocks; below 0.8 blocks per resident slot the
+    next smaller one is taken (pair likelihood, 1,000 x 256: 50 us with 250
+    tiles of 1024, 56 with 125 of 2048; 12 x 256: 30 us at 256, 34 at 512).
+    """
+    third, pair = nparams >= 14, precision == "pair"
+    if kind == "grad" and third:
+        return 512                    # its FP32 sums follow the tile
+    if precision == "fp64":
+        most, slots = 512, 2 * sms
+    else:
+        blocks = 2 if pair or kind == "grad" else 3
+        channels = 3 if kind == "wave" else 2
+        if kind == "grad":
+            bytes_ = 40
+        else:
+            bytes_ = 60 if third else channels * (16 if pair else 8)
+        most, slots = 4096, blocks * sms
+        while most > 512 and most * bytes_ > (76, 113)[blocks == 2] * 1024:
+            most //= 2
+    least = 2 if kind == "swap" else 1
+    tile = most
+    while tile > 256:
+        tiles = 0
+        for n, c in counts:
+            p = min(_MAX_PACK, max(least, tile // n))
+            tiles += -(-c // p)
+        if tiles >= 0.8 * slots:
+            break
+        tile //= 2
+    return tile
+
+
 class WavePlan:
     """Device-resident description of a batch (orbit tables, tiles, queue)."""
 
@@ -233,6 +278,8 @@ class GBGPUBase(abc.ABC):
         self._tables = {}
         self._plans = {}
         self._shapes = {}
+        self._sms = None
+        self._tiles = {}
         self._n_last = None
         self._status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._lazy = None
@@ -390,7 +437,8 @@ class GBGPUBase(abc.ABC):
         self.num_bin = B
         self.N = N
         self.df = 1 / T
-        plan = self._plan(N, T, precision, tdi2, params.shape[0])
+        plan = self._plan(N, T, precision, tdi2, params.shape[0],
+                          self._tile("wave", precision, params.shape[0], N, B))
         XYZ = torch.empty((B, 3, N), dtype=torch.complex128, device=self.device)
         AET = torch.empty((B, 3, N), dtype=torch.complex128, device=self.device)
         start = torch.empty(B, dtype=torch.int32, device=self.device)
@@ -548,11 +596,11 @@ class GBGPUBase(abc.ABC):
 
     def _launch_shape(self, kind, N, B, precision, tdi2, nparams, run, nkey=None, trusted=True):
         """(tile, blocks_per_sm) for this workload: the autotuner's choice when
-        autotuning is on (timing ``run`` on the first call), else defaults.
-        An unverified ``nkey`` (``trusted=False``) only looks up a cached
-        shape; a shape tuned now is filed under the contents' own key."""
-        if not self.autotune:
-            return 0, 0
+        autotuning is on (timing ``run`` on the first call), else the rule of
+        ``default_tile``.  An unverified ``nkey`` (``trusted=False``) only looks
+        up a cached shape; a new one is filed under the contents' own key."""
+        if not self.autotune and np.ndim(N) == 0:
+            return self._tile(kind, precision, nparams, N, B), 0
         if nkey is None:
             nkey = int(N) if np.ndim(N) == 0 else _array_key(np.ascontiguousarray(N, dtype=np.int64))
         ck = (kind, nkey, int(B), precision, bool(tdi2), int(nparams))
@@ -562,10 +610,35 @@ class GBGPUBase(abc.ABC):
             ck = (kind, nkey, int(B), precision, bool(tdi2), int(nparams))
             shape = self._shapes.get(ck)
         if shape is None:
-            from .autotune import default_tuner, workload_key
-            shape = default_tuner().tune(workload_key(kind, N, B, precision, tdi2, nparams), run)
+            if self.autotune:
+                from .autotune import default_tuner, workload_key
+                shape = default_tuner().tune(workload_key(kind, N, B, precision, tdi2, nparams), run)
+            else:
+                shape = self._tile(kind, precision, nparams, N, B), 0
+            while len(self._shapes) >= 4 * _PLAN_CACHE:
+                self._shapes.pop(next(iter(self._shapes)))
             self._shapes[ck] = shape
         return shape
+
+    def _tile(self, kind, precision, nparams, N, B):
+        """``default_tile`` for N (or one N per binary) on this device."""
+        key = None
+        if np.ndim(N) == 0:
+            counts = ((int(N), int(B)),)
+            key = (kind, precision, nparams, counts)
+            tile = self._tiles.get(key)
+            if tile is not None:
+                return tile
+        else:
+            counts = [(int(n), int(c)) for n, c in zip(*np.unique(N, return_counts=True))]
+        if self._sms is None:
+            self._sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        tile = default_tile(kind, precision, int(nparams), counts, self._sms)
+        if key is not None:
+            while len(self._tiles) >= 4 * _PLAN_CACHE:
+                self._tiles.pop(next(iter(self._tiles)))
+            self._tiles[key] = tile
+        return tile
 
     @staticmethod
     def _ll_args(dd, pp, data_length, data_index, noise_index, T):
@@ -769,15 +842,17 @@ class GBGPUBase(abc.ABC):
         if B:
             la = self._ll_args(dd, pp, L, di, ni, T)
 
+            nkey = None if np.ndim(N) == 0 else _array_key(N)
+
             def run(tile, bps):
-                plan = self._plan(N, T, "mixed", tdi2, npar, tile, bps)
+                plan = self._plan(N, T, "mixed", tdi2, npar, tile, bps, nkey=nkey)
                 a = plan.args(prm, start_freq_ind, self._status, grad=True)
                 rc = nat.lib().gbx_waveform_ll_grad(ctypes.byref(a), ctypes.byref(la),
                                                     nat.ptr(d_h), nat.ptr(h_h), nat.ptr(grad),
                                                     nat.stream_handle())
                 nat.check(rc, "gbx_waveform_ll_grad")
 
-            shape = self._launch_shape("grad", N, B, "mixed", tdi2, npar, run)
+            shape = self._launch_shape("grad", N, B, "mixed", tdi2, npar, run, nkey=nkey)
             self._status.zero_()
             run(*shape)
         self._lazy = (prm, N, T, tdi2)
@@ -836,7 +911,8 @@ class GBGPUBase(abc.ABC):
         out = torch.empty(B, dtype=torch.float64, device=self.device)
         gout = torch.zeros((self.NPARAMS, B), dtype=torch.float64, device=self.device) if grad else None
         if B:
-            plan = self._plan(N, T, precision, tdi2, self.NPARAMS)
+            plan = self._plan(N, T, precision, tdi2, self.NPARAMS,
+                              self._tile("grad" if grad else "swap", precision, self.NPARAMS, N, 2 * B))
             self._status.zero_()
             a = plan.args(prm, start_freq_ind, self._status, grad=grad)
             la = nat.LLArgs()
@@ -996,7 +1072,8 @@ class GBGPUBase(abc.ABC):
             AET = torch.empty((B, 3, int(N)), dtype=torch.complex128, device=self.device)
             start = torch.empty(B, dtype=torch.int32, device=self.device)
             if B:
-                plan = self._plan(N, T, precision, tdi2, prm.shape[0])
+                plan = self._plan(N, T, precision, tdi2, prm.shape[0],
+                                  self._tile("wave", precision, prm.shape[0], N, B))
                 a = plan.args(prm, start_freq_ind, self._status)
                 rc = nat.lib().gbx_waveform(ctypes.byref(a), None, nat.ptr(AET), nat.ptr(start),
                                             nat.stream_handle())
@@ -1008,7 +1085,8 @@ class GBGPUBase(abc.ABC):
         work[:, 0:2].zero_()
         self._status.zero_()
         if B:
-            plan = self._plan(N, T, precision, tdi2, prm.shape[0], self._fill_tile(N, sort))
+            plan = self._plan(N, T, precision, tdi2, prm.shape[0],
+                              self._fill_tile(N, sort, precision, prm))
             a = plan.args(prm, start_freq_ind, self._status)
             if sort:
                 self._fill_order(a, prm, gi, T, N)
@@ -1057,7 +1135,8 @@ class GBGPUBase(abc.ABC):
         B = params.shape[1]
         if B == 0:
             return
-        plan = self._plan(N, T, precision, tdi2, params.shape[0], self._fill_tile(N, sort))
+        plan = self._plan(N, T, precision, tdi2, params.shape[0],
+                          self._fill_tile(N, sort, precision, params))
         a = plan.args(params, start_freq_ind, self._status)
         if sort:
             self._fill_order(a, params, group_index, T, N)
@@ -1067,12 +1146,12 @@ class GBGPUBase(abc.ABC):
             nat.stream_handle())
         nat.check(rc, "gbx_waveform_fill")
 
-    @staticmethod
-    def _fill_tile(N, sort):
+    def _fill_tile(self, N, sort, precision, prm):
         """Samples per tile of a fill: sorted fills pack up to 16 binaries (at
-        most 4096 samples) so that neighbours share a tile; else the default."""
+        most 4096 samples) so that neighbours share a tile; else the rule of
+        ``default_tile``."""
         if not sort or np.ndim(N) != 0:
-            return 0
+            return self._tile("fill", precision, prm.shape[0], N, prm.shape[1])
         return int(min(16 * int(N), 4096))
 
     @staticmethod
