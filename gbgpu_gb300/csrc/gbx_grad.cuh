@@ -28,23 +28,18 @@ struct __align__(16) GradExtra {
     float cosvarpi, P2yr;          // third body: cos varpi, period in years
 };
 
-__device__ void setup_grad(GradExtra &X, const KParams &K, int b)
+__device__ void setup_grad(GradExtra &X, const KParams &K, int b, const Trig &t)
 {
     const gbx_wave_args &a = K.a;
     const int nb = a.num_bin;
     const double *p = a.params;
     double f0 = p[nb + b], fdot = p[2 * nb + b], fddot = p[3 * nb + b];
-    double iota = p[5 * nb + b], psi = p[6 * nb + b], lam = p[7 * nb + b], beta = p[8 * nb + b];
-    double theta = kPi / 2.0 - beta;
-    double st, ct, sp, cp, si, ci, s2p, c2p;
-    sincos(theta, &st, &ct);
-    sincos(lam, &sp, &cp);
-    sincos(iota, &si, &ci);
-    sincos(2.0 * psi, &s2p, &c2p);
-    X.u[0] = (float)(ct * cp); X.u[1] = (float)(ct * sp); X.u[2] = (float)(-st);
-    X.v[0] = (float)sp; X.v[1] = (float)(-cp); X.v[2] = 0.0f;
-    X.st = (float)st;
-    X.ct = (float)ct;
+    const double st = t.st, ct = t.ct, sp = t.sp, cp = t.cp, si = t.si, ci = t.ci;
+    const double s2p = t.s2p, c2p = t.c2p;
+    X.st = d2f_scaled(st, 0);
+    X.ct = d2f_scaled(ct, 0);
+    X.u[0] = d2f_scaled(ct * cp, 0); X.u[1] = d2f_scaled(ct * sp, 0); X.u[2] = -X.st;
+    X.v[0] = d2f_scaled(sp, 0); X.v[1] = d2f_scaled(-cp, 0); X.v[2] = 0.0f;
     // DP = Ap c2p - i Ac s2p, DC = -Ap s2p - i Ac c2p; Ap = 1 + ci^2, Ac = -2 ci
     const double Ap = 1.0 + ci * ci, Ac = -2.0 * ci;
     const double dAp = -2.0 * ci * si, dAc = 2.0 * si;
@@ -59,8 +54,8 @@ __device__ void setup_grad(GradExtra &X, const KParams &K, int b)
         const double wL = c * f0;
         X.dlnsc_f0 = make_double2(2.0 * c * cos(2.0 * wL) / sin(2.0 * wL), -2.0 * c);
     }
-    X.gf0 = (float)(-fdot / K.fstar);
-    X.gf1 = (float)(-fddot / K.fstar);
+    X.gf0 = d2f_scaled(-fdot * K.ifstar, 0);
+    X.gf1 = d2f_scaled(-fddot * K.ifstar, 0);
     X.cosvarpi = 0.0f;
     X.P2yr = 1.0f;
     if (a.nparams >= 14) {
@@ -877,8 +872,8 @@ __global__ void __launch_bounds__(kPrepBlock) prep_grad_kernel(const KParams K)
             memset(&sg[threadIdx.x], 0, sizeof(GradExtra));
             sb[threadIdx.x].b = -1;
         } else {
-            setup_bin(sb[threadIdx.x], K, b, 1 << lg, MODE_LL);
-            setup_grad(sg[threadIdx.x], K, b);
+            const Trig t = setup_bin(sb[threadIdx.x], K, b, 1 << lg, MODE_LL);
+            setup_grad(sg[threadIdx.x], K, b, t);
         }
     }
     __syncthreads();

@@ -69,7 +69,6 @@ struct __align__(16) Bin {
             dfl ap4, ci;
         } pr;
     };
-    double2 DP, DC;                // polarisation factors divided by amp
     double2 scale;                 // amp * 0.5 T / N [* tdi2 factor]
     union { double n2; dfl n2d; }; // n2 [rad/s]: FP64 form / float pair (mixed form)
     union { double T2; dfl T2d; }; // T2 [s], likewise
@@ -118,7 +117,7 @@ struct KParams {
     int num_groups;
     long long gstride;             // elements between consecutive groups of A_glob / E_glob
     int P;                         // binaries per tile in uniform mode
-    double fstar;                  // c / (2 pi L)
+    double fstar, ifstar;          // c / (2 pi L) and its reciprocal
     dfl stepd[GBX_MAX_LOG2N + 1];  // T / 2^k as float pairs (exact: division by a power of two)
     dfl Locd;                      // L / c as a float pair (pair form)
     double Loc;                    // L / c (FP64 form)
@@ -402,253 +401,7 @@ __device__ float vlos_grad_mixed(dfl t, const Bin &B, float cosvarpi, float P2yr
 }
 
 // ----------------------------------------------------------------------------
-// per-binary set-up (gbgpu.py:212-266, 296-309)
-// ----------------------------------------------------------------------------
-__device__ void setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
-{
-    const gbx_wave_args &a = K.a;
-    const int nb = a.num_bin;
-    const double *p = a.params;
-    double amp = p[b], f0 = p[nb + b], fdot = p[2 * nb + b], fddot = p[3 * nb + b];
-    double phi0 = p[4 * nb + b], iota = p[5 * nb + b], psi = p[6 * nb + b];
-    double lam = p[7 * nb + b], beta = p[8 * nb + b];
-    const double T = a.T;
-    B.b = b;
-    B.valid = 1;
-    B.f0 = f0; B.fdot = fdot; B.fddot = fddot;
-    {
-        // phi0 mod 2 pi: less rounding in the sums it enters (FP64 form)
-        const double k = rint(phi0 * kInvTwoPi);
-        B.phi0 = fma(-k, kTwoPiLo, fma(-k, kTwoPi, phi0));
-    }
-    double q = rint(f0 * T);
-    // om - 2 pi q/T cancels about seven digits; the two products are rounded
-    // separately (no FMA contraction) so the phase slope carries the same
-    // rounding as the reference's (om - df) (gbgpu.py:462-464, 497)
-    B.om = __dmul_rn(2.0 * kPi, f0);
-    B.om_m_dfa = __dsub_rn(B.om, __dmul_rn(2.0 * kPi, q / T));
-    B.pifdot = kPi * fdot;
-    B.pi3fddot = (1.0 / 3.0 * kPi) * fddot;
-    double ci = cos(iota);
-    double s1p, c1p;
-    sincos(psi, &s1p, &c1p);
-    const double s2p = 2.0 * s1p * c1p, c2p = fma(-2.0 * s1p, s1p, 1.0);
-    double Ap = 1.0 + ci * ci, Ac = -2.0 * ci;
-    B.DP = make_double2(Ap * c2p, -Ac * s2p);
-    B.DC = make_double2(-Ap * s2p, -Ac * c2p);
-    double theta = kPi / 2.0 - beta;
-    double st, ct, sp, cp;
-    sincos(theta, &st, &ct);
-    sincos(lam, &sp, &cp);
-    double u[3] = {ct * cp, ct * sp, -st};
-    double v[3] = {sp, -cp, 0.0};
-    B.k[0] = -st * cp; B.k[1] = -st * sp; B.k[2] = -ct;
-    // r.e+.r DP + r.ex.r DC = (r.v + i r.u)^2 with its real part times
-    // 1 + cos^2 iota and its imaginary part times 2 cos iota after a turn by
-    // 2 psi: the turn goes into the basis, v' + i u' = (v + i u) e^{i psi}
-    double vp[3], up[3];
-    for (int c = 0; c < 3; c++) {
-        vp[c] = v[c] * c1p - u[c] * s1p;
-        up[c] = v[c] * s1p + u[c] * c1p;
-    }
-    if (a.precision == GBX_PAIR) {
-        for (int c = 0; c < 3; c++) {
-            B.pr.up[c] = df_from(up[c]);
-            B.pr.vp[c] = df_from(vp[c]);
-        }
-        B.pr.ap4 = df_from(0.25 * Ap);
-        B.pr.ci = df_from(ci);
-    } else if (a.precision == GBX_FP64) {
-        for (int c = 0; c < 3; c++) {
-            B.q.up[c] = up[c];
-            B.q.vp[c] = vp[c];
-        }
-        B.q.ap4 = 0.25 * Ap;
-        B.q.ci = ci;
-        B.q.pf2 = 2.0 * B.pifdot;
-        B.q.p3f3 = 3.0 * B.pi3fddot;
-        for (int c = 0; c < 2; c++) {
-            B.q.kh[c] = rint(B.k[c] * 67108864.0) * (1.0 / 67108864.0);
-            B.q.kl[c] = B.k[c] - B.q.kh[c];
-        }
-    }
-    for (int c = 0; c < 3; c++) {
-        if (a.precision != GBX_FP64) {
-            B.kf[c] = (float)B.k[c];
-            B.uf[c] = (float)u[c];
-            B.vf[c] = (float)v[c];
-        }
-        B.kd[c] = df_from(B.k[c]);
-    }
-    B.omd = df_from(B.om);
-    B.omdfad = df_from(B.om_m_dfa);
-    B.phi0d = df_from(phi0);
-    B.pfd = df_from(B.pifdot);
-    B.tpfd = df_from(2.0 * B.pifdot);
-    B.p3d = df_from(B.pi3fddot);
-    B.pfddd = df_from(kPi * fddot);
-    B.DPf = make_float2((float)B.DP.x, (float)B.DP.y);
-    B.DCf = make_float2((float)B.DC.x, (float)B.DC.y);
-    B.f0f = (float)f0; B.fdotf = (float)fdot; B.fddotf = (float)fddot;
-    {
-        // f/fstar with the constant term kept as an unevaluated float pair so
-        // the FP32 transfer frequency carries no per-binary rounding bias
-        const double fstar = K.fstar;
-        double w0 = f0 / fstar;
-        B.w0h = (float)w0;
-        B.w0l = (float)(w0 - (double)B.w0h);
-        const double w1 = fdot / fstar;
-        B.w1 = (float)w1;
-        B.w1l = (float)(w1 - (double)B.w1);
-        B.w2 = (float)(0.5 * fddot / fstar);
-    }
-    // start index, bit-exact with round(((q - N/2)/T)/(1/T))  (gbgpu.py:296, 387)
-    double fmin = (q - (double)N / 2.0) / T;
-    double kmin = rint(fmin / (1.0 / T));
-    B.start = (int)kmin - a.start_freq_ind;
-    // output scaling (gbgpu.py:298-309): amp * 0.5 T / N [* 2i sin 2wL e^{-2iwL}]
-    double fc = 0.5 * T / (double)N;
-    double2 sc = make_double2(amp * fc, 0.0);
-    if (a.tdi2 == GBX_TDI2_BIT) {
-        double omL = 2.0 * kPi * f0 * (a.armlength / kCSI);
-        double s2, c2;
-        sincos(2.0 * omL, &s2, &c2);
-        // 2i s (c - i s) = 2 s^2 + 2i s c
-        double2 t2 = make_double2(2.0 * s2 * s2, 2.0 * s2 * c2);
-        sc = make_double2(fc * t2.x * amp, fc * t2.y * amp);
-    }
-    B.scale = sc;
-    if (a.nparams >= 14) {
-        const double A2 = p[9 * nb + b], varpi = p[10 * nb + b], e2 = p[11 * nb + b];
-        double P2 = p[12 * nb + b];
-        const double n2 = 2.0 * kPi / (P2 * a.year), T2 = p[13 * nb + b] * a.year;
-        if (a.precision == GBX_FP64) {
-            B.n2 = n2;
-            B.T2 = T2;
-            // A2 [sin(phi + varpi) + e sin varpi] with the true anomaly
-            // phi = u + 2 arg(1 - bt e^{-iu}), bt = (1 - sqrt(1 - e^2))/e
-            // (gbgpu/thirdbody.py:339-380), that is sin phi = sq sin u/(1 - eD cos u),
-            // cos phi = (cos u - eD)/(1 - eD cos u) with eD = 2 bt/(1 + bt^2) and
-            // sq = (1 - bt^2)/(1 + bt^2): eD is e up to bt's rounding, which
-            // reaches 1e-10 for small e and is kept as the model has it.  Below
-            // e = 1e-6 the model takes phi = u: bt = 0.
-            double sv, cv;
-            sincos(varpi, &sv, &cv);
-            const double bt = e2 > 1e-6 ? (1.0 - sqrt(1.0 - e2 * e2)) / e2 : 0.0;
-            const double ib = 1.0 / fma(bt, bt, 1.0), eD = 2.0 * bt * ib, sq = (1.0 - bt) * (1.0 + bt) * ib;
-            B.kep.e2 = e2;
-            B.kep.eD = eD;
-            B.kep.ka = A2 * (sq * cv);
-            B.kep.kb = A2 * (sq * sq * sv);                       // 1 - eD^2 = sq^2
-            B.kep.kc = A2 * ((e2 - eD) * sv);
-        } else {
-            B.n2d = df_from(n2);
-            B.T2d = df_from(T2);
-        }
-        B.A2f = (float)A2;
-        B.e2f = (float)e2;
-        double vr = varpi - 2.0 * kPi * floor(varpi * kInvTwoPi);
-        B.varpif = (float)vr;
-        B.sinvarpif = (float)sin(varpi);
-    }
-    B.di = B.ni = B.gi = 0;
-    B.eS = B.eD = 0;
-    if (mode == MODE_LL || mode == MODE_SWAP) {
-        int di = K.data_index ? K.data_index[b] : 0;
-        int ni = K.noise_index ? K.noise_index[b] : 0;
-        if (di < 0 || di >= K.num_data || ni < 0 || ni >= K.num_psd) {
-            flag(a.status, GBX_FLAG_INDEX);
-            B.valid = 0;
-            di = ni = 0;
-        }
-        B.di = di; B.ni = ni;
-        // power-of-two scalings so that S*2^eS and d*2^eD are O(1) in FP32
-        int jm = B.start + N / 2;
-        jm = jm < 0 ? 0 : (jm >= K.L ? K.L - 1 : jm);
-        double Sm = K.A_psd[(size_t)ni * K.L + jm];
-        int lg = (Sm > 0.0 && isfinite(Sm)) ? ilogb(Sm) : 0;
-        B.eS = -lg;
-        B.eD = -(lg >> 1) - 14;
-    } else if (mode == MODE_FILL) {
-        int gi = K.group_index[b];
-        if (gi < 0 || gi >= K.num_groups) {
-            flag(a.status, GBX_FLAG_INDEX);
-            B.valid = 0;
-            gi = 0;
-        }
-        B.gi = gi;
-        // a zero amplitude adds nothing (the samplers zero rejected proposals)
-        if (amp == 0.0) B.valid = 0;
-    }
-}
-
-// ----------------------------------------------------------------------------
-// Unequal arms (no counterpart in the reference, whose TDI assumes one
-// armlength, gbgpu.py:167-170): arm a = 12, 23, 31 has length ell_a L at the
-// sample, ell_a = |r_a| with r_a = (P_j - P_i)/L from the orbit table.  Each
-// link carries its own arm: transfer argument a = (f/f*)(ell_a +- k.r_a)/2 (the
-// reference's (f/f*)(1 +- k.r)/2 times ell_a with r normalised), antenna
-// pattern r.e.r / ell_a^2 and amplitude ell_a; the TDI delays are the phase
-// factors D_a = exp(-i omL ell_a) at the instantaneous frequency
-// (quasi-static: the slow part is not re-sampled at the delayed times):
-//   X = -2i omL [(1 - D_31^2)(G21 + D_12 G12) - (1 - D_12^2)(G31 + D_31 G13)]
-// with Y, Z cyclic, and TDI-2 multiplies X by (1 - D_12^2 D_31^2) (Y, Z
-// cyclic).  With every ell_a = 1 this is the reference's fctr2 [G21 - G31 +
-// (G12 - G13) fctr] (gbgpu.py:362-372), since -2i omL (1 - D^2) = 4 omL
-// sin(omL) e^{-i omL}, and its TDI-2 factor 1 - D^4 = 2i sin 2wL e^{-2iwL}
-// (gbgpu.py:298-309) evaluated at f(t) instead of f0.
-// ----------------------------------------------------------------------------
-__device__ __forceinline__ double2 one_minus(double2 z) { return make_double2(1.0 - z.x, -z.y); }
-
-__device__ __forceinline__ void slow_unequal_fp64(const Bin &B, double tm, double fstar,
-                                               const double (&r)[3][3], const double (&kdotr)[3],
-                                               const double (&fonfs)[3], const double (&kp)[3],
-                                               const double2 (&A)[3], int tdi, double2 out[3])
-{
-    double ell[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) ell[a] = sqrt(r[a][0] * r[a][0] + r[a][1] * r[a][1] + r[a][2] * r[a][2]);
-    double2 G[6];
-    const int arm[6] = {0, 1, 2, 0, 1, 2};
-    const int sc[6] = {0, 1, 2, 1, 2, 0};
-    const double sg[6] = {1.0, 1.0, 1.0, -1.0, -1.0, -1.0};
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        const double arg = 0.5 * fonfs[sc[q]] * (ell[arm[q]] + sg[q] * kdotr[arm[q]]);
-        double sn, cs;
-        sincos(arg + kp[sc[q]], &sn, &cs);
-        const double amp = 0.25 * sin(arg) / arg / ell[arm[q]];
-        G[q] = cmul(make_double2(amp * cs, -amp * sn), A[arm[q]]);
-    }
-    const double f = B.f0 + B.fdot * tm + 0.5 * B.fddot * tm * tm;
-    const double omL = f / fstar;
-    double2 D[3], D2[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        double sn, cs;
-        sincos(omL * ell[a], &sn, &cs);
-        D[a] = make_double2(cs, -sn);
-        D2[a] = cmul(D[a], D[a]);
-    }
-    double2 X = csub(cmul(one_minus(D2[2]), cadd(G[3], cmul(D[0], G[0]))),
-                     cmul(one_minus(D2[0]), cadd(G[2], cmul(D[2], G[5]))));
-    double2 Y = csub(cmul(one_minus(D2[0]), cadd(G[4], cmul(D[1], G[1]))),
-                     cmul(one_minus(D2[1]), cadd(G[0], cmul(D[0], G[3]))));
-    double2 Z = csub(cmul(one_minus(D2[1]), cadd(G[5], cmul(D[2], G[2]))),
-                     cmul(one_minus(D2[2]), cadd(G[1], cmul(D[1], G[4]))));
-    if (tdi & GBX_TDI2_BIT) {
-        X = cmul(one_minus(cmul(D2[0], D2[2])), X);
-        Y = cmul(one_minus(cmul(D2[1], D2[0])), Y);
-        Z = cmul(one_minus(cmul(D2[2], D2[1])), Z);
-    }
-    const double2 pre = make_double2(0.0, -2.0 * omL);
-    out[0] = cmul(pre, X);
-    out[1] = cmul(pre, Y);
-    out[2] = cmul(pre, Z);
-}
-
-// ----------------------------------------------------------------------------
-// FP64 slow part (gbgpu.py:399-540 and 348-375).  One FP64 warp instruction
+// FP64 arithmetic of the set-up and the FP64 form.  One FP64 warp instruction
 // occupies its scheduler's FP64 unit for 64 cycles (measured), against one
 // cycle for an FP32 one, so the form is bound by the number of FP64
 // instructions and everything below is arranged to need few of them: 381 per
@@ -730,6 +483,269 @@ __device__ __forceinline__ double recip_fp64(double x)
     return fma(fma(-x, r, 1.0), r, r);
 }
 
+// df_from with one FP64 instruction instead of four (the casts run on the FP64
+// pipe too): parts below FP32's normal range become zero
+__device__ __forceinline__ dfl df_split(double x)
+{
+    if ((__double2hiint(x) & 0x7ff00000) == 0x7ff00000) return df_from(x);
+    const float h = d2f_scaled(x, 0);
+    return {h, d2f_scaled(x - f2d_bits(h), 0)};
+}
+
+// ----------------------------------------------------------------------------
+// per-binary set-up (gbgpu.py:212-266, 296-309)
+// ----------------------------------------------------------------------------
+struct Trig {
+    double st, ct, sp, cp, si, ci, s2p, c2p;    // polar angle, lam, iota, 2 psi
+};
+
+// Bound by its FP64 instructions: with the table's sincos, one-instruction
+// splits into pairs and products with reciprocals from the host a warp takes 198
+// in the pair form (280 with the library's sincos, casts and divisions) and 213
+// in the mixed one (307): 40 -> 30 us for 50,000 binaries, and with the
+// gradient's part, which takes over the sines and cosines, 23 -> 16 us for 8,191.
+__device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
+{
+    const gbx_wave_args &a = K.a;
+    const int nb = a.num_bin;
+    const double *p = a.params;
+    double amp = p[b], f0 = p[nb + b], fdot = p[2 * nb + b], fddot = p[3 * nb + b];
+    double phi0 = p[4 * nb + b], iota = p[5 * nb + b], psi = p[6 * nb + b];
+    double lam = p[7 * nb + b], beta = p[8 * nb + b];
+    const double T = a.T;
+    B.b = b;
+    B.valid = 1;
+    B.f0 = f0; B.fdot = fdot; B.fddot = fddot;
+    {
+        // phi0 mod 2 pi: less rounding in the sums it enters (FP64 form)
+        const double k = rint(phi0 * kInvTwoPi);
+        B.phi0 = fma(-k, kTwoPiLo, fma(-k, kTwoPi, phi0));
+    }
+    double q = rint(f0 * T);
+    // om - 2 pi q/T cancels about seven digits; the two products are rounded
+    // separately (no FMA contraction) so the phase slope carries the same
+    // rounding as the reference's (om - df) (gbgpu.py:462-464, 497)
+    B.om = __dmul_rn(2.0 * kPi, f0);
+    B.om_m_dfa = __dsub_rn(B.om, __dmul_rn(2.0 * kPi, q / T));
+    B.pifdot = kPi * fdot;
+    B.pi3fddot = (1.0 / 3.0 * kPi) * fddot;
+    double si, ci, s1p, c1p;
+    sincos_tab(iota, g_sc_d, si, ci);
+    sincos_tab(psi, g_sc_d, s1p, c1p);
+    const double s2p = 2.0 * s1p * c1p, c2p = fma(-2.0 * s1p, s1p, 1.0);
+    double Ap = 1.0 + ci * ci, Ac = -2.0 * ci;
+    double theta = kPi / 2.0 - beta;
+    double st, ct, sp, cp;
+    sincos_tab(theta, g_sc_d, st, ct);
+    sincos_tab(lam, g_sc_d, sp, cp);
+    double u[3] = {ct * cp, ct * sp, -st};
+    double v[3] = {sp, -cp, 0.0};
+    B.k[0] = -st * cp; B.k[1] = -st * sp; B.k[2] = -ct;
+    // r.e+.r DP + r.ex.r DC = (r.v + i r.u)^2 with its real part times
+    // 1 + cos^2 iota and its imaginary part times 2 cos iota after a turn by
+    // 2 psi: the turn goes into the basis, v' + i u' = (v + i u) e^{i psi}
+    double vp[3], up[3];
+    for (int c = 0; c < 3; c++) {
+        vp[c] = v[c] * c1p - u[c] * s1p;
+        up[c] = v[c] * s1p + u[c] * c1p;
+    }
+    if (a.precision == GBX_PAIR) {
+        for (int c = 0; c < 3; c++) {
+            B.pr.up[c] = df_split(up[c]);
+            B.pr.vp[c] = df_split(vp[c]);
+        }
+        B.pr.ap4 = df_split(0.25 * Ap);
+        B.pr.ci = df_split(ci);
+    } else if (a.precision == GBX_FP64) {
+        for (int c = 0; c < 3; c++) {
+            B.q.up[c] = up[c];
+            B.q.vp[c] = vp[c];
+        }
+        B.q.ap4 = 0.25 * Ap;
+        B.q.ci = ci;
+        B.q.pf2 = 2.0 * B.pifdot;
+        B.q.p3f3 = 3.0 * B.pi3fddot;
+        for (int c = 0; c < 2; c++) {
+            B.q.kh[c] = rint(B.k[c] * 67108864.0) * (1.0 / 67108864.0);
+            B.q.kl[c] = B.k[c] - B.q.kh[c];
+        }
+    }
+    B.fdotf = d2f_scaled(fdot, 0);
+    B.fddotf = d2f_scaled(fddot, 0);
+    if (a.precision != GBX_FP64) {
+        for (int c = 0; c < 3; c++) {
+            B.kf[c] = d2f_scaled(B.k[c], 0);
+            B.uf[c] = d2f_scaled(u[c], 0);
+            B.vf[c] = d2f_scaled(v[c], 0);
+            B.kd[c] = df_split(B.k[c]);
+        }
+        B.omd = df_split(B.om);
+        B.omdfad = df_split(B.om_m_dfa);
+        B.phi0d = df_split(phi0);
+        B.pfd = df_split(B.pifdot);
+        B.tpfd = dfl{2.0f * B.pfd.h, 2.0f * B.pfd.l};
+        B.p3d = df_split(B.pi3fddot);
+        B.pfddd = df_split(kPi * fddot);
+        B.DPf = make_float2(d2f_scaled(Ap * c2p, 0), d2f_scaled(-Ac * s2p, 0));
+        B.DCf = make_float2(d2f_scaled(-Ap * s2p, 0), d2f_scaled(-Ac * c2p, 0));
+        B.f0f = d2f_scaled(f0, 0);
+        // f/fstar with the constant term kept as an unevaluated float pair so
+        // the FP32 transfer frequency carries no per-binary rounding bias
+        const dfl w0 = df_split(f0 * K.ifstar), w1 = df_split(fdot * K.ifstar);
+        B.w0h = w0.h;
+        B.w0l = w0.l;
+        B.w1 = w1.h;
+        B.w1l = w1.l;
+        B.w2 = d2f_scaled(0.5 * fddot * K.ifstar, 0);
+    }
+    // start index: round(((q - N/2)/T)/(1/T)) (gbgpu.py:296, 387) is q - N/2, the
+    // three roundings moving it by less than 1e-7 of a bin
+    B.start = (int)(q - (double)(N >> 1)) - a.start_freq_ind;
+    // output scaling (gbgpu.py:298-309): amp * 0.5 T / N [* 2i sin 2wL e^{-2iwL}]
+    double fc = 0.5 * T * exp2_int(__clz(N) - 31);           // 0.5 T / N
+    double2 sc = make_double2(amp * fc, 0.0);
+    if (a.tdi2 == GBX_TDI2_BIT) {
+        double omL = 2.0 * kPi * f0 * (a.armlength / kCSI);
+        double s2, c2;
+        sincos(2.0 * omL, &s2, &c2);
+        // 2i s (c - i s) = 2 s^2 + 2i s c
+        double2 t2 = make_double2(2.0 * s2 * s2, 2.0 * s2 * c2);
+        sc = make_double2(fc * t2.x * amp, fc * t2.y * amp);
+    }
+    B.scale = sc;
+    if (a.nparams >= 14) {
+        const double A2 = p[9 * nb + b], varpi = p[10 * nb + b], e2 = p[11 * nb + b];
+        double P2 = p[12 * nb + b];
+        const double n2 = 2.0 * kPi / (P2 * a.year), T2 = p[13 * nb + b] * a.year;
+        if (a.precision == GBX_FP64) {
+            B.n2 = n2;
+            B.T2 = T2;
+            // A2 [sin(phi + varpi) + e sin varpi] with the true anomaly
+            // phi = u + 2 arg(1 - bt e^{-iu}), bt = (1 - sqrt(1 - e^2))/e
+            // (gbgpu/thirdbody.py:339-380), that is sin phi = sq sin u/(1 - eD cos u),
+            // cos phi = (cos u - eD)/(1 - eD cos u) with eD = 2 bt/(1 + bt^2) and
+            // sq = (1 - bt^2)/(1 + bt^2): eD is e up to bt's rounding, which
+            // reaches 1e-10 for small e and is kept as the model has it.  Below
+            // e = 1e-6 the model takes phi = u: bt = 0.
+            double sv, cv;
+            sincos_tab(varpi, g_sc_d, sv, cv);
+            const double bt = e2 > 1e-6 ? (1.0 - sqrt(1.0 - e2 * e2)) / e2 : 0.0;
+            const double ib = 1.0 / fma(bt, bt, 1.0), eD = 2.0 * bt * ib, sq = (1.0 - bt) * (1.0 + bt) * ib;
+            B.kep.e2 = e2;
+            B.kep.eD = eD;
+            B.kep.ka = A2 * (sq * cv);
+            B.kep.kb = A2 * (sq * sq * sv);                       // 1 - eD^2 = sq^2
+            B.kep.kc = A2 * ((e2 - eD) * sv);
+        } else {
+            B.n2d = df_split(n2);
+            B.T2d = df_split(T2);
+            B.A2f = (float)A2;
+            double vr = varpi - 2.0 * kPi * floor(varpi * kInvTwoPi);
+            B.varpif = (float)vr;
+            B.sinvarpif = (float)sin(varpi);
+        }
+        B.e2f = (float)e2;
+    }
+    B.di = B.ni = B.gi = 0;
+    B.eS = B.eD = 0;
+    if (mode == MODE_LL || mode == MODE_SWAP) {
+        int di = K.data_index ? K.data_index[b] : 0;
+        int ni = K.noise_index ? K.noise_index[b] : 0;
+        if (di < 0 || di >= K.num_data || ni < 0 || ni >= K.num_psd) {
+            flag(a.status, GBX_FLAG_INDEX);
+            B.valid = 0;
+            di = ni = 0;
+        }
+        B.di = di; B.ni = ni;
+        // power-of-two scalings so that S*2^eS and d*2^eD are O(1) in FP32
+        int jm = B.start + N / 2;
+        jm = jm < 0 ? 0 : (jm >= K.L ? K.L - 1 : jm);
+        double Sm = K.A_psd[(size_t)ni * K.L + jm];
+        int lg = (Sm > 0.0 && isfinite(Sm)) ? ilogb(Sm) : 0;
+        B.eS = -lg;
+        B.eD = -(lg >> 1) - 14;
+    } else if (mode == MODE_FILL) {
+        int gi = K.group_index[b];
+        if (gi < 0 || gi >= K.num_groups) {
+            flag(a.status, GBX_FLAG_INDEX);
+            B.valid = 0;
+            gi = 0;
+        }
+        B.gi = gi;
+        // a zero amplitude adds nothing (the samplers zero rejected proposals)
+        if (amp == 0.0) B.valid = 0;
+    }
+    return Trig{st, ct, sp, cp, si, ci, s2p, c2p};
+}
+
+// ----------------------------------------------------------------------------
+// Unequal arms (no counterpart in the reference, whose TDI assumes one
+// armlength, gbgpu.py:167-170): arm a = 12, 23, 31 has length ell_a L at the
+// sample, ell_a = |r_a| with r_a = (P_j - P_i)/L from the orbit table.  Each
+// link carries its own arm: transfer argument a = (f/f*)(ell_a +- k.r_a)/2 (the
+// reference's (f/f*)(1 +- k.r)/2 times ell_a with r normalised), antenna
+// pattern r.e.r / ell_a^2 and amplitude ell_a; the TDI delays are the phase
+// factors D_a = exp(-i omL ell_a) at the instantaneous frequency
+// (quasi-static: the slow part is not re-sampled at the delayed times):
+//   X = -2i omL [(1 - D_31^2)(G21 + D_12 G12) - (1 - D_12^2)(G31 + D_31 G13)]
+// with Y, Z cyclic, and TDI-2 multiplies X by (1 - D_12^2 D_31^2) (Y, Z
+// cyclic).  With every ell_a = 1 this is the reference's fctr2 [G21 - G31 +
+// (G12 - G13) fctr] (gbgpu.py:362-372), since -2i omL (1 - D^2) = 4 omL
+// sin(omL) e^{-i omL}, and its TDI-2 factor 1 - D^4 = 2i sin 2wL e^{-2iwL}
+// (gbgpu.py:298-309) evaluated at f(t) instead of f0.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ double2 one_minus(double2 z) { return make_double2(1.0 - z.x, -z.y); }
+
+__device__ __forceinline__ void slow_unequal_fp64(const Bin &B, double tm, double fstar,
+                                               const double (&r)[3][3], const double (&kdotr)[3],
+                                               const double (&fonfs)[3], const double (&kp)[3],
+                                               const double2 (&A)[3], int tdi, double2 out[3])
+{
+    double ell[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) ell[a] = sqrt(r[a][0] * r[a][0] + r[a][1] * r[a][1] + r[a][2] * r[a][2]);
+    double2 G[6];
+    const int arm[6] = {0, 1, 2, 0, 1, 2};
+    const int sc[6] = {0, 1, 2, 1, 2, 0};
+    const double sg[6] = {1.0, 1.0, 1.0, -1.0, -1.0, -1.0};
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        const double arg = 0.5 * fonfs[sc[q]] * (ell[arm[q]] + sg[q] * kdotr[arm[q]]);
+        double sn, cs;
+        sincos(arg + kp[sc[q]], &sn, &cs);
+        const double amp = 0.25 * sin(arg) / arg / ell[arm[q]];
+        G[q] = cmul(make_double2(amp * cs, -amp * sn), A[arm[q]]);
+    }
+    const double f = B.f0 + B.fdot * tm + 0.5 * B.fddot * tm * tm;
+    const double omL = f / fstar;
+    double2 D[3], D2[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        double sn, cs;
+        sincos(omL * ell[a], &sn, &cs);
+        D[a] = make_double2(cs, -sn);
+        D2[a] = cmul(D[a], D[a]);
+    }
+    double2 X = csub(cmul(one_minus(D2[2]), cadd(G[3], cmul(D[0], G[0]))),
+                     cmul(one_minus(D2[0]), cadd(G[2], cmul(D[2], G[5]))));
+    double2 Y = csub(cmul(one_minus(D2[0]), cadd(G[4], cmul(D[1], G[1]))),
+                     cmul(one_minus(D2[1]), cadd(G[0], cmul(D[0], G[3]))));
+    double2 Z = csub(cmul(one_minus(D2[1]), cadd(G[5], cmul(D[2], G[2]))),
+                     cmul(one_minus(D2[2]), cadd(G[1], cmul(D[1], G[4]))));
+    if (tdi & GBX_TDI2_BIT) {
+        X = cmul(one_minus(cmul(D2[0], D2[2])), X);
+        Y = cmul(one_minus(cmul(D2[1], D2[0])), Y);
+        Z = cmul(one_minus(cmul(D2[2], D2[1])), Z);
+    }
+    const double2 pre = make_double2(0.0, -2.0 * omL);
+    out[0] = cmul(pre, X);
+    out[1] = cmul(pre, Y);
+    out[2] = cmul(pre, Z);
+}
+
+// ----------------------------------------------------------------------------
+// FP64 slow part (gbgpu.py:399-540 and 348-375)
+// ----------------------------------------------------------------------------
 // The general path, used with unequal arms: every link with its own carrier.
 __device__ __forceinline__ void slow_links_fp64(const Bin &B, int n, int N, double tm, int tdi,
                                              const double *__restrict__ tab, double fstar,
@@ -2334,6 +2350,7 @@ static KParams base_params(const gbx_wave_args *a)
     memset(&K, 0, sizeof(K));
     K.a = *a;
     K.fstar = kCSI / (a->armlength * 2.0 * kPi);
+    K.ifstar = 1.0 / K.fstar;
     for (int k = 0; k <= GBX_MAX_LOG2N; k++) K.stepd[k] = df_from(ldexp(a->T, -k));
     K.Locd = df_from(a->armlength / kCSI);
     K.Loc = a->armlength / kCSI;
