@@ -36,10 +36,10 @@ __device__ void setup_grad(GradExtra &X, const KParams &K, int b, const Trig &t)
     double f0 = p[nb + b], fdot = p[2 * nb + b], fddot = p[3 * nb + b];
     const double st = t.st, ct = t.ct, sp = t.sp, cp = t.cp, si = t.si, ci = t.ci;
     const double s2p = t.s2p, c2p = t.c2p;
-    X.st = d2f_scaled(st, 0);
-    X.ct = d2f_scaled(ct, 0);
-    X.u[0] = d2f_scaled(ct * cp, 0); X.u[1] = d2f_scaled(ct * sp, 0); X.u[2] = -X.st;
-    X.v[0] = d2f_scaled(sp, 0); X.v[1] = d2f_scaled(-cp, 0); X.v[2] = 0.0f;
+    X.st = d2f_rn(st);
+    X.ct = d2f_rn(ct);
+    X.u[0] = d2f_rn(ct * cp); X.u[1] = d2f_rn(ct * sp); X.u[2] = -X.st;
+    X.v[0] = d2f_rn(sp); X.v[1] = d2f_rn(-cp); X.v[2] = 0.0f;
     // DP = Ap c2p - i Ac s2p, DC = -Ap s2p - i Ac c2p; Ap = 1 + ci^2, Ac = -2 ci
     const double Ap = 1.0 + ci * ci, Ac = -2.0 * ci;
     const double dAp = -2.0 * ci * si, dAc = 2.0 * si;
@@ -54,8 +54,8 @@ __device__ void setup_grad(GradExtra &X, const KParams &K, int b, const Trig &t)
         const double wL = c * f0;
         X.dlnsc_f0 = make_double2(2.0 * c * cos(2.0 * wL) / sin(2.0 * wL), -2.0 * c);
     }
-    X.gf0 = d2f_scaled(-fdot * K.ifstar, 0);
-    X.gf1 = d2f_scaled(-fddot * K.ifstar, 0);
+    X.gf0 = d2f_rn(-fdot / K.fstar);
+    X.gf1 = d2f_rn(-fddot / K.fstar);
     X.cosvarpi = 0.0f;
     X.P2yr = 1.0f;
     if (a.nparams >= 14) {

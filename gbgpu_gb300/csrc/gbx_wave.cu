@@ -269,6 +269,18 @@ __device__ __forceinline__ float d2f_scaled(double x, int e)
     return __uint_as_float((hi & 0x80000000u) | (mag & 0x7fffffffu));
 }
 
+// the same with ties to even and no scaling: (float)x for values in FP32's
+// normal range, zero below it
+__device__ __forceinline__ float d2f_rn(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int ne = (int)((hi >> 20) & 0x7ffu) - 896;
+    unsigned mag = __funnelshift_l(lo, hi, 3) - (896u << 23) +
+                   ((lo >> 28) & ((lo & 0x2fffffffu) != 0u ? 1u : 0u));
+    mag = ((unsigned)(ne - 1) < 254u) ? mag : (ne >= 255 ? 0x7f800000u : 0u);
+    return __uint_as_float((hi & 0x80000000u) | (mag & 0x7fffffffu));
+}
+
 // FP32 -> FP64 (exact) on the integer pipe: exponent rebias, mantissa shift;
 // FP32 zeros and subnormals give signed zero, infinities stay infinite.
 __device__ __forceinline__ double f2d_bits(float f)
@@ -488,8 +500,8 @@ __device__ __forceinline__ double recip_fp64(double x)
 __device__ __forceinline__ dfl df_split(double x)
 {
     if ((__double2hiint(x) & 0x7ff00000) == 0x7ff00000) return df_from(x);
-    const float h = d2f_scaled(x, 0);
-    return {h, d2f_scaled(x - f2d_bits(h), 0)};
+    const float h = d2f_rn(x);
+    return {h, d2f_rn(x - f2d_bits(h))};
 }
 
 // ----------------------------------------------------------------------------
@@ -499,11 +511,21 @@ struct Trig {
     double st, ct, sp, cp, si, ci, s2p, c2p;    // polar angle, lam, iota, 2 psi
 };
 
+// the library's sincos, out of line
+__device__ __noinline__ double2 sincos_lib(double x)
+{
+    double s, c;
+    sincos(x, &s, &c);
+    return make_double2(s, c);
+}
+
 // Bound by its FP64 instructions: with the table's sincos, one-instruction
 // splits into pairs and products with reciprocals from the host a warp takes 198
-// in the pair form (280 with the library's sincos, casts and divisions) and 213
-// in the mixed one (307): 40 -> 30 us for 50,000 binaries, and with the
-// gradient's part, which takes over the sines and cosines, 23 -> 16 us for 8,191.
+// in the pair form, 280 with the library's sincos, casts and divisions (17 -> 11
+// us for 1,000 binaries in the FP64 form).  The mixed form keeps the library's
+// sincos and the divisions: another last bit there moves an FP32 rounding in one
+// window of 10^5, by up to 4e-7 of a gradient; its splits alone take a warp
+// from 307 to 265 (50,000 binaries 40 -> 37 us, gradient 8,191 23 -> 19 us).
 __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
 {
     const gbx_wave_args &a = K.a;
@@ -529,15 +551,25 @@ __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     B.om_m_dfa = __dsub_rn(B.om, __dmul_rn(2.0 * kPi, q / T));
     B.pifdot = kPi * fdot;
     B.pi3fddot = (1.0 / 3.0 * kPi) * fddot;
+    const bool lib = a.precision == GBX_MIXED;
+    auto sc_of = [lib](double x, double &s, double &c) {
+        if (lib) {
+            const double2 r = sincos_lib(x);
+            s = r.x;
+            c = r.y;
+        } else {
+            sincos_tab(x, g_sc_d, s, c);
+        }
+    };
     double si, ci, s1p, c1p;
-    sincos_tab(iota, g_sc_d, si, ci);
-    sincos_tab(psi, g_sc_d, s1p, c1p);
+    sc_of(iota, si, ci);
+    sc_of(psi, s1p, c1p);
     const double s2p = 2.0 * s1p * c1p, c2p = fma(-2.0 * s1p, s1p, 1.0);
     double Ap = 1.0 + ci * ci, Ac = -2.0 * ci;
     double theta = kPi / 2.0 - beta;
     double st, ct, sp, cp;
-    sincos_tab(theta, g_sc_d, st, ct);
-    sincos_tab(lam, g_sc_d, sp, cp);
+    sc_of(theta, st, ct);
+    sc_of(lam, sp, cp);
     double u[3] = {ct * cp, ct * sp, -st};
     double v[3] = {sp, -cp, 0.0};
     B.k[0] = -st * cp; B.k[1] = -st * sp; B.k[2] = -ct;
@@ -570,13 +602,13 @@ __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
             B.q.kl[c] = B.k[c] - B.q.kh[c];
         }
     }
-    B.fdotf = d2f_scaled(fdot, 0);
-    B.fddotf = d2f_scaled(fddot, 0);
+    B.fdotf = d2f_rn(fdot);
+    B.fddotf = d2f_rn(fddot);
     if (a.precision != GBX_FP64) {
         for (int c = 0; c < 3; c++) {
-            B.kf[c] = d2f_scaled(B.k[c], 0);
-            B.uf[c] = d2f_scaled(u[c], 0);
-            B.vf[c] = d2f_scaled(v[c], 0);
+            B.kf[c] = d2f_rn(B.k[c]);
+            B.uf[c] = d2f_rn(u[c]);
+            B.vf[c] = d2f_rn(v[c]);
             B.kd[c] = df_split(B.k[c]);
         }
         B.omd = df_split(B.om);
@@ -586,17 +618,18 @@ __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
         B.tpfd = dfl{2.0f * B.pfd.h, 2.0f * B.pfd.l};
         B.p3d = df_split(B.pi3fddot);
         B.pfddd = df_split(kPi * fddot);
-        B.DPf = make_float2(d2f_scaled(Ap * c2p, 0), d2f_scaled(-Ac * s2p, 0));
-        B.DCf = make_float2(d2f_scaled(-Ap * s2p, 0), d2f_scaled(-Ac * c2p, 0));
-        B.f0f = d2f_scaled(f0, 0);
+        B.DPf = make_float2(d2f_rn(Ap * c2p), d2f_rn(-Ac * s2p));
+        B.DCf = make_float2(d2f_rn(-Ap * s2p), d2f_rn(-Ac * c2p));
+        B.f0f = d2f_rn(f0);
         // f/fstar with the constant term kept as an unevaluated float pair so
         // the FP32 transfer frequency carries no per-binary rounding bias
-        const dfl w0 = df_split(f0 * K.ifstar), w1 = df_split(fdot * K.ifstar);
+        const dfl w0 = df_split(lib ? f0 / K.fstar : f0 * K.ifstar);
+        const dfl w1 = df_split(lib ? fdot / K.fstar : fdot * K.ifstar);
         B.w0h = w0.h;
         B.w0l = w0.l;
         B.w1 = w1.h;
         B.w1l = w1.l;
-        B.w2 = d2f_scaled(0.5 * fddot * K.ifstar, 0);
+        B.w2 = d2f_rn(lib ? 0.5 * fddot / K.fstar : 0.5 * fddot * K.ifstar);
     }
     // start index: round(((q - N/2)/T)/(1/T)) (gbgpu.py:296, 387) is q - N/2, the
     // three roundings moving it by less than 1e-7 of a bin
