@@ -29,6 +29,7 @@ EXPORTS = (
     "gbx_waveform", "gbx_waveform_ll", "gbx_waveform_fill", "gbx_wave_workspace_bytes",
     "gbx_waveform_ll_noalloc", "gbx_waveform_ll_grad", "gbx_grad_workspace_bytes",
     "gbx_swap_ll", "gbx_swap_ll_grad", "gbx_fisher", "gbx_fill_global_det", "gbx_math_selftest",
+    "gbx_log_likelihood",
 )
 
 _vp = ctypes.c_void_p
@@ -88,6 +89,8 @@ def lib():
     L.gbx_wave_workspace_bytes.restype = ctypes.c_size_t
     L.gbx_waveform.argtypes = [ctypes.POINTER(WaveArgs), _vp, _vp, _vp, _vp]
     L.gbx_waveform_ll.argtypes = [ctypes.POINTER(WaveArgs), ctypes.POINTER(LLArgs), _vp, _vp, _vp]
+    L.gbx_log_likelihood.argtypes = [ctypes.POINTER(WaveArgs), ctypes.POINTER(LLArgs), _vp, _vp,
+                                     _d, _vp, _vp]
     L.gbx_waveform_ll_noalloc.argtypes = [ctypes.POINTER(WaveArgs), ctypes.POINTER(LLArgs),
                                           _vp, _vp, _vp]
     L.gbx_waveform_ll_grad.argtypes = [ctypes.POINTER(WaveArgs), ctypes.POINTER(LLArgs),

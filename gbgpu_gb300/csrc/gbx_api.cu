@@ -68,6 +68,55 @@ int ensure_init(cudaStream_t st)
 
 extern "C" int gbx_version(void) { return 100; }
 
+// The attributes a kernel needs and its occupancy are properties of (kernel,
+// device, block, shared memory), so they are set and asked for once each: three
+// driver calls less per launch (about 5 us of a small call).  A larger dynamic
+// shared memory limit serves smaller launches too, so it only grows.
+int kernel_fit(const void *kern, int block, size_t smem, int *per_sm)
+{
+    struct Entry {
+        const void *kern;
+        size_t smem;
+        int dev, block, per_sm;
+    };
+    constexpr int kEntries = 128;
+    static std::mutex lock;
+    static Entry table[kEntries];
+    static int used = 0, next = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_error(e, "cudaGetDevice");
+    if (smem > 227 * 1024) return set_error(GBX_ERR_UNSUPPORTED, "tile needs %zu B of shared memory", smem);
+    std::lock_guard<std::mutex> g(lock);
+    size_t limit = 0;
+    for (int k = 0; k < used; k++) {
+        const Entry &t = table[k];
+        if (t.kern != kern || t.dev != dev) continue;
+        if (t.smem == smem && t.block == block) {
+            *per_sm = t.per_sm;
+            return GBX_OK;
+        }
+        limit = t.smem > limit ? t.smem : limit;
+    }
+    if (smem > limit || limit == 0) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute");
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(carveout)");
+    }
+    int n = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem);
+    if (e != cudaSuccess) return cuda_error(e, "occupancy");
+    *per_sm = n;
+    // full: the oldest entry goes; its kernel's limit stands at least as high
+    // as the entries left say, which at worst sets it again
+    table[next] = Entry{kern, smem, dev, block, n};
+    next = (next + 1) % kEntries;
+    used = used < kEntries ? used + 1 : used;
+    return GBX_OK;
+}
+
 extern "C" const char *gbx_last_error(void) { return g_msg; }
 
 extern "C" int gbx_init(void) { return ensure_init(0); }

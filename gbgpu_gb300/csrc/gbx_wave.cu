@@ -2255,15 +2255,10 @@ static size_t pair_smem_bytes(int maxS, int nch, int maxP)
 template <int MODE>
 static int launch_tiles(void (*kern)(const KParams), size_t sm, const KParams &K, cudaStream_t st)
 {
-    if (sm > 227 * 1024) return set_error(GBX_ERR_UNSUPPORTED, "tile needs %zu B of shared memory", sm);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute");
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(carveout)");
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, sm);
-    if (e != cudaSuccess) return cuda_error(e, "occupancy");
+    int rc = kernel_fit((const void *)kern, kBlock, sm, &per_sm);
+    if (rc) return rc;
+    cudaError_t e;
     if (K.a.blocks_per_sm > 0 && per_sm > K.a.blocks_per_sm) per_sm = K.a.blocks_per_sm;
     if (per_sm < 1) per_sm = 1;
     int nsm = num_sms();
@@ -2278,8 +2273,9 @@ static int launch_tiles(void (*kern)(const KParams), size_t sm, const KParams &K
     if (K.a.workspace) {
         const size_t psm = sizeof(Bin) * kPrepBlock;
         auto pk = prep_kernel<MODE>;
-        e = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-        if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(prep)");
+        int unused = 0;
+        rc = kernel_fit((const void *)pk, kPrepBlock, psm, &unused);
+        if (rc) return rc;
         pk<<<(K.a.num_bin + kPrepBlock - 1) / kPrepBlock, kPrepBlock, psm, st>>>(K);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_error(e, "prep_kernel launch");
@@ -2573,15 +2569,10 @@ static int launch_grad(const gbx_wave_args &b, const gbx_ll_args *l, void *d_h, 
     const bool third = b.nparams == 14;
     auto kern = third ? grad_kernel<true, SWAP> : grad_kernel<false, SWAP>;
     const size_t sm = grad_smem_bytes(third, maxS, K.maxP);
-    if (sm > 227 * 1024) return set_error(GBX_ERR_UNSUPPORTED, "tile needs %zu B of shared memory", sm);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(grad)");
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(grad carveout)");
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, sm);
-    if (e != cudaSuccess) return cuda_error(e, "occupancy(grad)");
+    int per_sm = 0, unused = 0;
+    int rc = kernel_fit((const void *)kern, kBlock, sm, &per_sm);
+    if (rc) return rc;
+    cudaError_t e;
     if (b.blocks_per_sm > 0 && per_sm > b.blocks_per_sm) per_sm = b.blocks_per_sm;
     if (per_sm < 1) per_sm = 1;
     const int ntiles = b.tiles ? b.ntiles : (b.num_bin + K.P - 1) / K.P;
@@ -2593,8 +2584,8 @@ static int launch_grad(const gbx_wave_args &b, const gbx_ll_args *l, void *d_h, 
         if (e != cudaSuccess) return cuda_error(e, "queue reset");
     }
     const size_t psm = (sizeof(Bin) + sizeof(GradExtra)) * kPrepBlock;
-    e = cudaFuncSetAttribute(prep_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(prep_grad)");
+    rc = kernel_fit((const void *)prep_grad_kernel, kPrepBlock, psm, &unused);
+    if (rc) return rc;
     prep_grad_kernel<<<(b.num_bin + kPrepBlock - 1) / kPrepBlock, kPrepBlock, psm, st>>>(K);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "prep_grad_kernel launch");
@@ -2686,14 +2677,10 @@ extern "C" int gbx_fisher(const gbx_wave_args *a, const double *A_psd, const dou
     F.fisher = fisher;
     const size_t sm = fisher_smem_bytes(maxS, K.maxP);
     if (sm > 227 * 1024) return set_error(GBX_ERR_UNSUPPORTED, "tile needs %zu B of shared memory (use a smaller tile)", sm);
-    cudaError_t e = cudaFuncSetAttribute(fisher_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(fisher)");
-    e = cudaFuncSetAttribute(fisher_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(fisher carveout)");
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fisher_kernel, kBlock, sm);
-    if (e != cudaSuccess) return cuda_error(e, "occupancy(fisher)");
+    int per_sm = 0, unused = 0;
+    rc = kernel_fit((const void *)fisher_kernel, kBlock, sm, &per_sm);
+    if (rc) return rc;
+    cudaError_t e;
     if (b.blocks_per_sm > 0 && per_sm > b.blocks_per_sm) per_sm = b.blocks_per_sm;
     if (per_sm < 1) per_sm = 1;
     const int ntiles = b.tiles ? b.ntiles : (b.num_bin + K.P - 1) / K.P;
@@ -2705,8 +2692,8 @@ extern "C" int gbx_fisher(const gbx_wave_args *a, const double *A_psd, const dou
         if (e != cudaSuccess) return cuda_error(e, "queue reset");
     }
     const size_t psm = (sizeof(Bin) + sizeof(GradExtra)) * kPrepBlock;
-    e = cudaFuncSetAttribute(prep_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(prep_grad)");
+    rc = kernel_fit((const void *)prep_grad_kernel, kPrepBlock, psm, &unused);
+    if (rc) return rc;
     prep_grad_kernel<<<(b.num_bin + kPrepBlock - 1) / kPrepBlock, kPrepBlock, psm, st>>>(K);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "prep_grad_kernel launch");
@@ -2714,6 +2701,38 @@ extern "C" int gbx_fisher(const gbx_wave_args *a, const double *A_psd, const dou
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "fisher_kernel launch");
     return GBX_OK;
+}
+
+// The end of a likelihood call on the device: logL from its terms and the
+// status word as one more number, so that the caller reads everything back in
+// one copy (instead of five elementwise launches and two copies).
+namespace gbx {
+__global__ void ll_finish_kernel(const double2 *d_h, const double2 *h_h, double d_d, int n,
+                                 const int *status, double *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the reference's order, -1/2 (d_d + h_h - 2 d_h) (gbgpu.py:728)
+    if (i < n) out[i] = -0.5 * __dsub_rn(__dadd_rn(d_d, h_h[i].x), 2.0 * d_h[i].x);
+    else if (i == n) out[n] = status ? (double)*status : 0.0;
+}
+}  // namespace gbx
+
+extern "C" int gbx_log_likelihood(const gbx_wave_args *a, const gbx_ll_args *l, void *d_h, void *h_h,
+                                  double d_d, double *out, void *stream)
+{
+    if (!a || !out) return set_error(GBX_ERR_ARG, "NULL wave args / output");
+    cudaStream_t st = (cudaStream_t)stream;
+    if (a->status) {
+        const cudaError_t e = cudaMemsetAsync(a->status, 0, sizeof(int), st);
+        if (e != cudaSuccess) return cuda_error(e, "status reset");
+    }
+    const int rc = gbx_waveform_ll(a, l, d_h, h_h, stream);
+    if (rc) return rc;
+    const int n = a->num_bin;
+    gbx::ll_finish_kernel<<<n / 256 + 1, 256, 0, st>>>((const double2 *)d_h, (const double2 *)h_h, d_d, n,
+                                                       a->status, out);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? GBX_OK : cuda_error(e, "ll_finish_kernel launch");
 }
 
 // ----------------------------------------------------------------------------

@@ -201,33 +201,38 @@ class WavePlan:
             self.tables[n.bit_length() - 1] = owner._orbit_table(n, self.T)
         self.queue = torch.zeros(1, dtype=torch.int32, device=dev) if not self.uniform else None
         self._ws = None
+        self._fixed = None
 
     def args(self, params, start_freq_ind=0, status=None, grad=False):
         """gbx_wave_args for this plan.  The struct holds references to the
         plan and to ``params`` so that the device buffers it points to (tile
         list, queue, workspace, orbit tables) live as long as it does."""
-        a = nat.WaveArgs()
+        if self._fixed is None:
+            # what does not change from call to call
+            a = nat.WaveArgs()
+            a.N = self.N
+            a.precision = _PRECISIONS[self.precision]
+            a.tdi2 = self.tdi2
+            a.T = self.T
+            a.year = YRSID_SI
+            for lg, t in self.tables.items():
+                a.orbit[lg] = t.data_ptr()
+            a.order = self.order.data_ptr() if self.order is not None else None
+            a.tiles = self.tiles.data_ptr() if self.tiles is not None else None
+            a.ntiles = self.ntiles
+            a.queue = self.queue.data_ptr() if self.queue is not None else None
+            a.tile = self.tile
+            a.blocks_per_sm = self.blocks_per_sm
+            self._fixed = a
+        a = nat.WaveArgs.from_buffer_copy(self._fixed)
         a._keep = (self, params, status)
         a.params = params.data_ptr()
-        a.num_bin = params.shape[1]
-        a.nparams = params.shape[0]
-        a.N = self.N
-        a.precision = _PRECISIONS[self.precision]
-        a.tdi2 = self.tdi2
+        a.nparams, B = params.shape
+        a.num_bin = B
         a.start_freq_ind = int(start_freq_ind)
-        a.T = self.T
         a.armlength = float(self.owner.orbits.armlength)
-        a.year = YRSID_SI
-        for lg, t in self.tables.items():
-            a.orbit[lg] = t.data_ptr()
-        a.order = self.order.data_ptr() if self.order is not None else None
-        a.tiles = self.tiles.data_ptr() if self.tiles is not None else None
-        a.ntiles = self.ntiles
-        a.queue = self.queue.data_ptr() if self.queue is not None else None
-        a.status = status.data_ptr() if status is not None else None
-        a.tile = self.tile
-        a.blocks_per_sm = self.blocks_per_sm
-        B = params.shape[1]
+        if status is not None:
+            a.status = status.data_ptr()
         need = (nat.lib().gbx_grad_workspace_bytes(B) if grad
                 else nat.lib().gbx_wave_workspace_bytes(B))
         if need:
@@ -394,6 +399,10 @@ class GBGPUBase(abc.ABC):
             base = _native(base)
         if isinstance(base, (np.ndarray, torch.Tensor)) and base.ndim == 2 and not add_args:
             return _to_device(base, torch.float64, self.device).contiguous()
+        rows = [*base, *add_args]
+        if all(isinstance(x, torch.Tensor) and x.ndim == 1 and x.dtype == torch.float64 and
+               x.device == self.device and x.shape == rows[0].shape for x in rows):
+            return torch.stack(rows)
         cols = [torch.atleast_1d(_to_device(x, torch.float64, self.device)) for x in base]
         B = cols[0].shape[0]
         rows = [c.expand(B) if c.shape[0] == 1 and B > 1 else c for c in cols]
@@ -581,17 +590,16 @@ class GBGPUBase(abc.ABC):
             raise ValueError("data must be 1-D or 2-D")
         dd = [_to_device(x, torch.complex128, self.device).reshape(-1).contiguous() for x in data]
         pp = [_to_device(x, torch.float64, self.device).reshape(-1).contiguous() for x in psd]
-        if data_index is None:
-            data_index = torch.zeros(num_bin, dtype=torch.int32, device=self.device)
-        if noise_index is None:
-            noise_index = torch.zeros(num_bin, dtype=torch.int32, device=self.device)
-        # reference checks (gbgpu.py:681-686)
-        assert len(data_index) == num_bin
-        assert len(data_index) == len(noise_index)
-        assert str(data_index.dtype).endswith("int32")
-        assert str(noise_index.dtype).endswith("int32")
-        data_index = _to_device(data_index, torch.int32, self.device).contiguous()
-        noise_index = _to_device(noise_index, torch.int32, self.device).contiguous()
+        # reference checks (gbgpu.py:681-686); no index means row 0, which the
+        # kernels take without an array of zeros
+        if data_index is not None:
+            assert len(data_index) == num_bin
+            assert str(data_index.dtype).endswith("int32")
+            data_index = _to_device(data_index, torch.int32, self.device).contiguous()
+        if noise_index is not None:
+            assert len(noise_index) == num_bin
+            assert str(noise_index.dtype).endswith("int32")
+            noise_index = _to_device(noise_index, torch.int32, self.device).contiguous()
         return dd, pp, data_length, data_index, noise_index
 
     def _launch_shape(self, kind, N, B, precision, tdi2, nparams, run, nkey=None, trusted=True):
@@ -649,13 +657,15 @@ class GBGPUBase(abc.ABC):
         la.data_length = int(data_length)
         la.num_data = int(dd[0].numel() // data_length)
         la.num_psd = int(pp[0].numel() // data_length)
-        la.data_index = data_index.data_ptr()
-        la.noise_index = noise_index.data_ptr()
+        la.data_index = data_index.data_ptr() if data_index is not None else None
+        la.noise_index = noise_index.data_ptr() if noise_index is not None else None
         la.df = 1.0 / T
         return la
 
     def _fused_ll(self, params, N, T, tdi2, dd, pp, data_length, data_index, noise_index,
-                  start_freq_ind, precision):
+                  start_freq_ind, precision, d_d, out):
+        """d_h and h_h (B,); ``out`` (B + 1,) gets the log-likelihoods for the
+        scalar ``d_d`` and the status word (gbx_log_likelihood)."""
         B = params.shape[1]
         d_h = torch.empty(B, dtype=torch.complex128, device=self.device)
         h_h = torch.empty(B, dtype=torch.complex128, device=self.device)
@@ -673,13 +683,13 @@ class GBGPUBase(abc.ABC):
             plan = self._plan(N, T, precision, tdi2, nparams, tile, bps, nkey=nkey,
                               trusted=not verify)
             a = plan.args(params, start_freq_ind, self._status)
-            rc = nat.lib().gbx_waveform_ll(ctypes.byref(a), ctypes.byref(la), nat.ptr(d_h),
-                                           nat.ptr(h_h), nat.stream_handle())
-            nat.check(rc, "gbx_waveform_ll")
+            rc = nat.lib().gbx_log_likelihood(ctypes.byref(a), ctypes.byref(la), nat.ptr(d_h),
+                                              nat.ptr(h_h), d_d, nat.ptr(out),
+                                              nat.stream_handle())
+            nat.check(rc, "gbx_log_likelihood")
 
         shape = self._launch_shape("ll", N, B, precision, tdi2, nparams, run, nkey=nkey,
                                    trusted=not verify)
-        self._status.zero_()
         run(*shape)
         if verify:
             # the full key, computed while the kernel runs; if the array changed
@@ -691,7 +701,6 @@ class GBGPUBase(abc.ABC):
             if full != nkey:
                 nkey = full
                 shape = self._launch_shape("ll", N, B, precision, tdi2, nparams, run, nkey=nkey)
-                self._status.zero_()
                 run(*shape)
         return d_h, h_h
 
@@ -711,8 +720,12 @@ class GBGPUBase(abc.ABC):
         self._n_last = (arr.ctypes.data, n, sample, key)
         return key, False
 
-    def _check_status(self):
-        st = int(self._status.item())
+    def _check_status(self, st=None):
+        """Raise or warn for the kernels' flags (``st``: the status word, read
+        back here when the caller does not have it)."""
+        st = int(self._status.item()) if st is None else int(st)
+        if not st:
+            return
         if st & nat.GBX_FLAG_INDEX:
             raise ValueError("a data/noise/group index is out of range")
         if st & nat.GBX_FLAG_WINDOW:
@@ -751,12 +764,11 @@ class GBGPUBase(abc.ABC):
                 params.shape[0] == self.NPARAMS:
             # get_ll reads the likelihood back before returning
             prm = _to_device(params, torch.float64, self.device, non_blocking=True).contiguous()
-            base = [params[0], params[1]]
             extra = [params[i] for i in range(9, self.NPARAMS)]
             if extra:
                 self.prepare_additional_args(*extra)
             if N is None:
-                N = self._resolve_N(N, base[0], base[1], T, extra, oversample)
+                N = self._resolve_N(N, params[0], params[1], T, extra, oversample)
             elif np.ndim(N) != 0:
                 N = np.asarray(_to_host(N), dtype=np.int64).reshape(-1)
             else:
@@ -772,21 +784,29 @@ class GBGPUBase(abc.ABC):
         self.N = N
         self.df = df = 1 / T
         dd, pp, L, di, ni = self._prepare_data(data, psd, data_index, noise_index, B)
-        d_h, h_h = self._fused_ll(prm, N, T, tdi2, dd, pp, L, di, ni, start_freq_ind, precision)
+        # a scalar d_d enters as a kernel argument, not a device copy
+        d_d = self.d_d if isinstance(self.d_d, (int, float)) else _to_host(self.d_d)
+        scalar = np.ndim(d_d) == 0
+        out = torch.zeros(1, dtype=torch.float64, device=self.device) if B == 0 else \
+            torch.empty(B + 1, dtype=torch.float64, device=self.device)
+        d_h, h_h = self._fused_ll(prm, N, T, tdi2, dd, pp, L, di, ni, start_freq_ind, precision,
+                                  float(d_d) if scalar else 0.0, out)
         self._lazy = (prm, N, T, tdi2)
         if phase_marginalize:
             self.non_marg_d_h = d_h.cpu().numpy().copy()
             d_h = torch.abs(d_h).to(torch.complex128)
         self.h_h = h_h
         self.d_h = d_h
-        # the reference's order, -1/2 (d_d + h_h - 2 d_h) (gbgpu.py:728); a
-        # scalar d_d enters as a kernel argument, not a device copy
-        d_d = float(self.d_d) if np.ndim(_to_host(self.d_d)) == 0 else \
-            torch.as_tensor(self.d_d, device=self.device)
+        if scalar and not phase_marginalize:
+            res = out.cpu().numpy()
+            self._check_status(res[B])
+            return res[:B]
+        # the reference's order, -1/2 (d_d + h_h - 2 d_h) (gbgpu.py:728)
+        d_d = float(d_d) if scalar else torch.as_tensor(self.d_d, device=self.device)
         like = -1.0 / 2.0 * (d_d + h_h - 2 * d_h).real
-        out = like.cpu().numpy()
+        res = like.cpu().numpy()
         self._check_status()
-        return out
+        return res
 
     def get_ll_grad(self, params, data, psd, start_freq_ind=0, data_index=None,
                     noise_index=None, **kwargs):
@@ -803,7 +823,8 @@ class GBGPUBase(abc.ABC):
                                            noise_index, **kwargs)
         if kwargs.get("return_tensors"):
             return like, grad
-        return like.cpu().numpy(), grad.cpu().numpy()
+        both = torch.cat([like[None], grad]).cpu().numpy()
+        return both[0], both[1:]
 
     def _ll_grad_tensors(self, params, data, psd, start_freq_ind=0, data_index=None,
                          noise_index=None, **kwargs):
@@ -857,8 +878,10 @@ class GBGPUBase(abc.ABC):
             run(*shape)
         self._lazy = (prm, N, T, tdi2)
         self.d_h, self.h_h = d_h, h_h
-        d_d = torch.as_tensor(self.d_d, device=self.device)
-        like = -0.5 * (d_d + h_h.real - 2 * d_h.real)
+        # (a Python number needs no device copy)
+        d_d = self.d_d if isinstance(self.d_d, (int, float)) else \
+            torch.as_tensor(self.d_d, device=self.device)
+        like = -0.5 * ((d_d + h_h.real).sub_(d_h.real, alpha=2))
         return like, grad
 
     def swap_likelihood(self, params_old, params_new, data, psd, start_freq_ind=0,
@@ -905,25 +928,19 @@ class GBGPUBase(abc.ABC):
         prm = torch.stack([po, pn], dim=2).reshape(self.NPARAMS, 2 * B).contiguous()
         di = None if data_index is None else _to_device(data_index, torch.int32, self.device)
         ni = None if noise_index is None else _to_device(noise_index, torch.int32, self.device)
-        di2 = None if di is None else di.repeat_interleave(2).contiguous()
-        ni2 = None if ni is None else ni.repeat_interleave(2).contiguous()
+        di2 = None if di is None else di[:, None].expand(-1, 2).reshape(-1)
+        ni2 = None if ni is None else ni[:, None].expand(-1, 2).reshape(-1)
         dd, pp, L, di2, ni2 = self._prepare_data(data, psd, di2, ni2, 2 * B)
-        out = torch.empty(B, dtype=torch.float64, device=self.device)
+        # (one number more for the status word: everything comes back in one copy)
+        buf = torch.empty(B + 1, dtype=torch.float64, device=self.device)
+        out = buf[:B]
         gout = torch.zeros((self.NPARAMS, B), dtype=torch.float64, device=self.device) if grad else None
         if B:
             plan = self._plan(N, T, precision, tdi2, self.NPARAMS,
                               self._tile("grad" if grad else "swap", precision, self.NPARAMS, N, 2 * B))
             self._status.zero_()
             a = plan.args(prm, start_freq_ind, self._status, grad=grad)
-            la = nat.LLArgs()
-            la.A_data, la.E_data = dd[0].data_ptr(), dd[1].data_ptr()
-            la.A_psd, la.E_psd = pp[0].data_ptr(), pp[1].data_ptr()
-            la.data_length = int(L)
-            la.num_data = int(dd[0].numel() // L)
-            la.num_psd = int(pp[0].numel() // L)
-            la.data_index = di2.data_ptr()
-            la.noise_index = ni2.data_ptr()
-            la.df = 1.0 / T
+            la = self._ll_args(dd, pp, L, di2, ni2, T)
             if grad:
                 rc = nat.lib().gbx_swap_ll_grad(ctypes.byref(a), ctypes.byref(la), nat.ptr(out),
                                                 nat.ptr(gout), nat.stream_handle())
@@ -934,9 +951,10 @@ class GBGPUBase(abc.ABC):
                 nat.check(rc, "gbx_swap_ll")
         if return_tensor:
             return (out, gout) if grad else out
-        res = out.cpu().numpy()
-        self._check_status()
-        return (res, gout.cpu().numpy()) if grad else res
+        buf[B:].copy_(self._status)
+        res = buf.cpu().numpy()
+        self._check_status(res[B])
+        return (res[:B], gout.cpu().numpy()) if grad else res[:B]
 
     # --------------------------------------------------------- global fill
     def fill_global_template(self, group_index, templates, A, E, start_inds, N=None,
@@ -1055,7 +1073,7 @@ class GBGPUBase(abc.ABC):
         base, extra = [pT[i] for i in range(9)], [pT[i] for i in range(9, pT.shape[0])]
         add_args = self.prepare_additional_args(*extra) if extra else ()
         N = self._resolve_N(N, base[0], base[1], T, extra, oversample)
-        prm = self._params(base, add_args)
+        prm = self._params(base, add_args) if extra else pT[:9].contiguous()
         B = prm.shape[1]
         self.num_bin, self.N, self.df = B, N, 1 / T
         total_groups, nchannels, data_length = templates.shape

@@ -264,6 +264,16 @@ int gbx_waveform_ll(const gbx_wave_args *a, const gbx_ll_args *l, void *d_h, voi
                     void *stream);
 
 /*
+ * gbx_waveform_ll and the end of get_ll (gbgpu.py:728) in one call: clears
+ * *a->status (when given), computes d_h and h_h, and writes
+ * out[b] = -1/2 (d_d + Re h_h[b] - 2 Re d_h[b]) for every binary and the status
+ * word after the kernels as out[num_bin], so that one copy of num_bin + 1
+ * doubles brings back everything.
+ */
+int gbx_log_likelihood(const gbx_wave_args *a, const gbx_ll_args *l, void *d_h, void *h_h,
+                       double d_d, double *out, void *stream);
+
+/*
  * Fused run_wave + fill_global (reference gbgpu/gbgpu.py:839-878): scatter-adds
  * A and E of every binary into A_glob/E_glob[group_index[b]*L + j] with FP64
  * atomics.  Group g starts at element g * group_stride (0 = data_length).
