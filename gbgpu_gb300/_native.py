@@ -21,6 +21,7 @@ GBX_TDI_UNEQUAL = 2
 GBX_FLAG_WINDOW = 1
 GBX_FLAG_INDEX = 2
 GBX_FLAG_TILE = 4
+GBX_FLAG_COPY = 8
 
 EXPORTS = (
     "gbx_version", "gbx_last_error", "gbx_device_info", "gbx_init",

@@ -182,6 +182,126 @@ __global__ void __launch_bounds__(256) fill_global_kernel(
     }
 }
 
+// Row-major templates (t_stride_i == 1): a binary's window is one contiguous run
+// of each template, so it goes through shared memory as bulk copies (TMA): one
+// lane of each warp copies chunks of up to kBulkBins bins in, and adds them to
+// the template with a bulk reduction (FP64 additions in L2).  No thread touches
+// the data, and a warp keeps kBulkStages chunks in flight.  Bound by HBM: 50,000
+// windows of 256 bins into 8 templates of 0.5 M bins move 0.91 GB (templates
+// read, sums read and written back) in 150 us, 6.1 TB/s; a warp per window with
+// four FP64 reductions per bin took 197 us waiting on their round trips (one
+// template, whose sums stay in L2: 168 -> 97 us).  64 to 512 bins a chunk, 3 to
+// 12 stages and 2 to 8 warps are within 5 %.
+constexpr int kBulkBins = 256, kBulkStages = 4, kBulkWarps = 2;
+constexpr size_t kBulkSmem = (size_t)kBulkWarps * kBulkStages * kBulkBins * sizeof(double2);
+constexpr int kBulkPolls = 1 << 20;      // bounded waits: far beyond any copy
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__global__ void __launch_bounds__(kBulkWarps * 32) fill_global_bulk_kernel(
+    double2 *__restrict__ A_g, double2 *__restrict__ E_g, const double2 *__restrict__ A_t,
+    const double2 *__restrict__ E_t, const int *__restrict__ start_ind, int M, int num_bin,
+    const int *__restrict__ group_index, int L, long long gstride, long long tsb, int num_groups,
+    int *status)
+{
+    extern __shared__ __align__(128) unsigned char bulk_smem[];
+    __shared__ __align__(8) unsigned long long bars[kBulkWarps][kBulkStages];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane != 0) return;
+    double2 *buf = reinterpret_cast<double2 *>(bulk_smem) + (size_t)warp * kBulkStages * kBulkBins;
+    for (int k = 0; k < kBulkStages; k++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bars[warp][k])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // Work items: chunk c of channel ch of binary b.  `get` walks this warp's
+    // items in order and skips what lies outside the data (gbgpu_utils.cu:88-91).
+    const int chunks = (M + kBulkBins - 1) / kBulkBins;
+    const int stride = gridDim.x * kBulkWarps;
+    int b = blockIdx.x * kBulkWarps + warp, c = 0, ch = 0;
+    struct Item {
+        const double2 *src;
+        double2 *dst;
+        unsigned bytes;
+    };
+    int s = 0;
+    long long goff = -1;
+    auto load_bin = [&]() {
+        goff = -1;
+        if (b >= num_bin) return;
+        s = start_ind[b];
+        const int g = group_index[b];
+        if (num_groups > 0 && (g < 0 || g >= num_groups)) flag(status, GBX_FLAG_INDEX);
+        else goff = (long long)g * gstride;
+    };
+    load_bin();
+    auto get = [&](Item &it) -> bool {
+        while (b < num_bin) {
+            const int i0 = c * kBulkBins, i1 = min(M, i0 + kBulkBins);
+            const long long lo = max((long long)i0, -(long long)s), hi = min((long long)i1, (long long)L - s);
+            const bool have = goff >= 0 && hi > lo;
+            if (have) {
+                it.src = (ch ? E_t : A_t) + (long long)b * tsb + lo;
+                it.dst = (ch ? E_g : A_g) + goff + s + lo;
+                it.bytes = (unsigned)(hi - lo) * (unsigned)sizeof(double2);
+            }
+            if (++ch == 2) {
+                ch = 0;
+                if (++c == chunks) {
+                    c = 0;
+                    b += stride;
+                    load_bin();
+                }
+            }
+            if (have) return true;
+        }
+        return false;
+    };
+    auto issue = [&](int k, const Item &it) {
+        const unsigned bar = smem_addr(&bars[warp][k]);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(it.bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_addr(buf + (size_t)k * kBulkBins)), "l"(it.src), "r"(it.bytes), "r"(bar) : "memory");
+    };
+    Item items[kBulkStages];
+    int in = 0;                          // copies issued
+    bool more = true;
+    // one stage stays free for the reduction that still reads its chunk
+#pragma unroll
+    for (int k = 0; k < kBulkStages - 1; k++) {
+        if (more && (more = get(items[k]))) {
+            issue(k, items[k]);
+            in++;
+        }
+    }
+    bool ok = true;
+    for (int done = 0; done < in;) {
+#pragma unroll
+        for (int k = 0; k < kBulkStages; k++) {
+            if (done >= in) break;
+            const unsigned parity = (unsigned)(done / kBulkStages) & 1u;
+            unsigned ready = 0;
+            for (int poll = 0; poll < kBulkPolls && !ready; poll++)
+                asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                             "selp.u32 %0, 1, 0, p;\n}" : "=r"(ready) : "r"(smem_addr(&bars[warp][k])), "r"(parity) : "memory");
+            ok = ok && ready;
+            if (ready)
+                asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(
+                                 items[k].dst), "r"(smem_addr(buf + (size_t)k * kBulkBins)), "r"(items[k].bytes) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            done++;
+            // the stage of the previous reduction: refill it once it has been read
+            const int kn = k == 0 ? kBulkStages - 1 : k - 1;
+            asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            if (more && (more = get(items[kn]))) {
+                issue(kn, items[kn]);
+                in++;
+            }
+        }
+    }
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (!ok) flag(status, GBX_FLAG_COPY);
+}
+
 // Point-major templates (t_stride_b == 1, the reference's i * num_bin + b):
 // one CTA per chunk of 32 binaries.  Slabs of 32 samples x 32 binaries are
 // read one row per warp instruction (512 contiguous bytes), transposed
@@ -409,7 +529,19 @@ extern "C" int gbx_fill_global_ex(void *A_glob, void *E_glob, const void *A_temp
     if (group_stride < data_length) return set_error(GBX_ERR_ARG, "group_stride < data_length");
     int rc = ensure_init((cudaStream_t)stream);
     if (rc) return rc;
-    if (t_stride_b == 1 && t_stride_i >= num_bin) {
+    if (t_stride_i == 1 && M >= 8 &&
+        (((uintptr_t)A_glob | (uintptr_t)E_glob | (uintptr_t)A_template | (uintptr_t)E_template) & 15) == 0) {
+        // row-major templates: bulk copies and reductions (windows of a few bins
+        // are not worth a copy each)
+        int per_sm = 0;
+        rc = kernel_fit((const void *)fill_global_bulk_kernel, kBulkWarps * 32, kBulkSmem, &per_sm);
+        if (rc) return rc;
+        const int need = (num_bin + kBulkWarps - 1) / kBulkWarps, cap = num_sms() * (per_sm > 0 ? per_sm : 1);
+        fill_global_bulk_kernel<<<need < cap ? need : cap, kBulkWarps * 32, kBulkSmem, (cudaStream_t)stream>>>(
+            (double2 *)A_glob, (double2 *)E_glob, (const double2 *)A_template,
+            (const double2 *)E_template, start_ind, M, num_bin, group_index, data_length,
+            group_stride, t_stride_b, num_groups, status);
+    } else if (t_stride_b == 1 && t_stride_i >= num_bin) {
         // point-major templates: coalesced slabs through shared memory
         const int chunks = (num_bin + 31) / 32;
         const int cap = num_sms() * 6;

@@ -1043,8 +1043,11 @@ class GBGPUBase(abc.ABC):
             templates[...] = tt.cpu().numpy()
         elif tt is not templates:
             templates.copy_(tt)
-        if int(self._status.item()) & nat.GBX_FLAG_INDEX:
+        st = int(self._status.item())
+        if st & nat.GBX_FLAG_INDEX:
             raise ValueError("group_index out of range")
+        if st & nat.GBX_FLAG_COPY:
+            raise RuntimeError("a bulk copy did not complete")
 
     def generate_global_template(self, params, group_index, templates, start_freq_ind=0,
                                  **kwargs):
