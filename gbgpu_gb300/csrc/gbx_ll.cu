@@ -31,6 +31,8 @@ __device__ __forceinline__ dfl pair_sum_df(dfl v)
     return v;
 }
 
+constexpr int kLlBlock = 128;
+
 // <d|h>, <h|h> per binary (gbgpu_utils.cu:124-210).  A warp takes two
 // binaries: lane 2q + t walks points q, q + 16, ... of binary b + t, so a
 // warp's template loads cover whole 32-byte sectors in the point-major layout
@@ -45,7 +47,7 @@ __device__ __forceinline__ dfl pair_sum_df(dfl v)
 // FP64: the same mapping with the reference's arithmetic, FP64 products and
 // sums (gbgpu_utils.cu:167-179, the division by S as a product with 1/S).
 template <bool FP64>
-__global__ void __launch_bounds__(256) get_ll_kernel(
+__global__ void __launch_bounds__(kLlBlock, 8) get_ll_kernel(
     double2 *__restrict__ d_h, double2 *__restrict__ h_h, const double2 *__restrict__ A_t,
     const double2 *__restrict__ E_t, const double2 *__restrict__ A_d,
     const double2 *__restrict__ E_d, const double *__restrict__ A_p,
@@ -98,31 +100,68 @@ __global__ void __launch_bounds__(256) get_ll_kernel(
                 xh += (hA.x * hA.x + hA.y * hA.y) * wA + (hE.x * hE.x + hE.y * hE.y) * wE;
             }
         }
-#pragma unroll 2
-        for (int i = q; i < (FP64 ? 0 : Mh); i += 16) {
-            const int j = s + i;
-            if (j < 0 || j >= L) {
-                out = true;
-                continue;
-            }
-            const double2 hA = __ldg(A_t + i * tsi + b * tsb);
-            const double2 hE = __ldg(E_t + i * tsi + b * tsb);
-            const double2 dA = __ldg(A_d + doff + j), dE = __ldg(E_d + doff + j);
-            dfl reA, imA, sqA, reE, imE, sqE;
-            ll_terms(dA, hA, eD, reA, imA, sqA);
-            ll_terms(dE, hE, eD, reE, imE, sqE);
-            // accumulators stay normalised
-            if (same) {
-                const dfl w = df_recip(d2ff_scaled(__ldg(A_p + noff + j), eS));
-                dr = df_add(dr, df_prod(df_sum(reA, reE), w));
-                di = df_add(di, df_prod(df_sum(imA, imE), w));
-                hh = df_add(hh, df_prod(df_sum(sqA, sqE), w));
+        if constexpr (!FP64) {
+            // one bin's products from its loaded values
+            auto bin = [&](double2 hA, double2 hE, double2 dA, double2 dE, double SA, double SE) {
+                dfl reA, imA, sqA, reE, imE, sqE;
+                ll_terms(dA, hA, eD, reA, imA, sqA);
+                ll_terms(dE, hE, eD, reE, imE, sqE);
+                // accumulators stay normalised
+                if (same) {
+                    const dfl w = df_recip(d2ff_scaled(SA, eS));
+                    dr = df_add(dr, df_prod(df_sum(reA, reE), w));
+                    di = df_add(di, df_prod(df_sum(imA, imE), w));
+                    hh = df_add(hh, df_prod(df_sum(sqA, sqE), w));
+                } else {
+                    const dfl wA = df_recip(d2ff_scaled(SA, eS));
+                    const dfl wE = df_recip(d2ff_scaled(SE, eS));
+                    dr = df_add(dr, df_sum(df_prod(reA, wA), df_prod(reE, wE)));
+                    di = df_add(di, df_sum(df_prod(imA, wA), df_prod(imE, wE)));
+                    hh = df_add(hh, df_sum(df_prod(sqA, wA), df_prod(sqE, wE)));
+                }
+            };
+            // A window inside the data (nearly all of them) needs no test per
+            // bin, so the next bin's loads are issued before this one's ~200
+            // instructions.  Bound by those (integer-pipe splits above all) and,
+            // still, by load latency: 50,000 x 256 205 -> 182 us, 3,000 x 2048
+            // 259 -> 120 (64 registers, 8 blocks of 128 per SM; 80 registers 184
+            // and 115).  Splitting without the range handling (10 instructions
+            // instead of 17) spills: 234 us.
+            if (s >= 0 && s <= L - Mh) {
+                const double2 *pA = A_t + (long long)q * tsi + b * tsb, *pE = E_t + (long long)q * tsi + b * tsb;
+                const double2 *qA = A_d + doff + s, *qE = E_d + doff + s;
+                const double *rA = A_p + noff + s, *rE = E_p + noff + s;
+                double2 hA, hE, dA, dE;
+                double SA = 0.0, SE = 0.0;
+                auto load = [&](int i) {
+                    hA = __ldg(pA);
+                    hE = __ldg(pE);
+                    pA += 16 * tsi;
+                    pE += 16 * tsi;
+                    dA = __ldg(qA + i);
+                    dE = __ldg(qE + i);
+                    SA = __ldg(rA + i);
+                    if (!same) SE = __ldg(rE + i);
+                };
+                int i = q;
+                if (i < Mh) load(i);
+                while (i < Mh) {
+                    const double2 tA = hA, tE = hE, uA = dA, uE = dE;
+                    const double vA = SA, vE = SE;
+                    i += 16;
+                    if (i < Mh) load(i);
+                    bin(tA, tE, uA, uE, vA, vE);
+                }
             } else {
-                const dfl wA = df_recip(d2ff_scaled(__ldg(A_p + noff + j), eS));
-                const dfl wE = df_recip(d2ff_scaled(__ldg(E_p + noff + j), eS));
-                dr = df_add(dr, df_sum(df_prod(reA, wA), df_prod(reE, wE)));
-                di = df_add(di, df_sum(df_prod(imA, wA), df_prod(imE, wE)));
-                hh = df_add(hh, df_sum(df_prod(sqA, wA), df_prod(sqE, wE)));
+                for (int i = q; i < Mh; i += 16) {
+                    const int j = s + i;
+                    if (j < 0 || j >= L) {
+                        out = true;
+                        continue;
+                    }
+                    bin(__ldg(A_t + i * tsi + b * tsb), __ldg(E_t + i * tsi + b * tsb), __ldg(A_d + doff + j),
+                        __ldg(E_d + doff + j), __ldg(A_p + noff + j), __ldg(E_p + noff + j));
+                }
             }
         }
         if constexpr (FP64) {
@@ -470,7 +509,10 @@ static int get_ll_launch(void *d_h, void *h_h, const void *A_template, const voi
         return set_error(GBX_ERR_ARG, "NULL pointer");
     int rc = ensure_init((cudaStream_t)stream);
     if (rc) return rc;
-    get_ll_kernel<FP64><<<grid_for((num_bin + 1) / 2), 256, 0, (cudaStream_t)stream>>>(
+    // one warp per pair of binaries, in small blocks (a grid-stride loop over the
+    // resident warps leaves the last of 2.6 rounds for 50,000 part empty)
+    const long long warps = ((long long)num_bin + 1) / 2, per = kLlBlock / 32;
+    get_ll_kernel<FP64><<<(unsigned)((warps + per - 1) / per), kLlBlock, 0, (cudaStream_t)stream>>>(
         (double2 *)d_h, (double2 *)h_h, (const double2 *)A_template, (const double2 *)E_template,
         (const double2 *)A_data, (const double2 *)E_data, A_psd, E_psd, df, start_ind, M, num_bin,
         data_index, noise_index, data_length, t_stride_i, t_stride_b, num_data, num_psd, status);
