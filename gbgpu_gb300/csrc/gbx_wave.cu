@@ -521,11 +521,12 @@ __device__ __noinline__ double2 sincos_lib(double x)
 
 // Bound by its FP64 instructions: with the table's sincos, one-instruction
 // splits into pairs and products with reciprocals from the host a warp takes 198
-// in the pair form, 280 with the library's sincos, casts and divisions (17 -> 11
-// us for 1,000 binaries in the FP64 form).  The mixed form keeps the library's
-// sincos and the divisions: another last bit there moves an FP32 rounding in one
-// window of 10^5, by up to 4e-7 of a gradient; its splits alone take a warp
-// from 307 to 265 (50,000 binaries 40 -> 37 us, gradient 8,191 23 -> 19 us).
+// in the pair form, 280 with the library's sincos, casts and divisions.  The
+// mixed and FP64 forms keep the library's sincos and the divisions: in the mixed
+// form another last bit moves an FP32 rounding in one window of 10^5, by up to
+// 4e-7 of a gradient (its splits alone take a warp from 307 to 265; 50,000
+// binaries 40 -> 37 us, gradient 8,191 23 -> 19 us), and in the FP64 form the last
+// bit of k, 5e-14 s of k.P, is as large as the form's other rounding errors.
 __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
 {
     const gbx_wave_args &a = K.a;
@@ -551,7 +552,7 @@ __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     B.om_m_dfa = __dsub_rn(B.om, __dmul_rn(2.0 * kPi, q / T));
     B.pifdot = kPi * fdot;
     B.pi3fddot = (1.0 / 3.0 * kPi) * fddot;
-    const bool lib = a.precision == GBX_MIXED;
+    const bool lib = a.precision != GBX_PAIR;
     auto sc_of = [lib](double x, double &s, double &c) {
         if (lib) {
             const double2 r = sincos_lib(x);
@@ -661,7 +662,7 @@ __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
             // reaches 1e-10 for small e and is kept as the model has it.  Below
             // e = 1e-6 the model takes phi = u: bt = 0.
             double sv, cv;
-            sincos_tab(varpi, g_sc_d, sv, cv);
+            sc_of(varpi, sv, cv);
             const double bt = e2 > 1e-6 ? (1.0 - sqrt(1.0 - e2 * e2)) / e2 : 0.0;
             const double ib = 1.0 / fma(bt, bt, 1.0), eD = 2.0 * bt * ib, sq = (1.0 - bt) * (1.0 + bt) * ib;
             B.kep.e2 = e2;
@@ -912,7 +913,19 @@ __device__ __forceinline__ void slow_fp64(const Bin &B, int n, int N, double tm,
     // |d| < 1e-9 everywhere (|k.r| <= 1): high word of dd below that of 5e-10
     const bool tiny = !THIRD && (__double2hiint(dd) & 0x7fffffff) < 0x3e012e0b;
     double sh, ch;
-    sincos_tab(h, sct, sh, ch);
+    if ((__double2hiint(h) & 0x7fffffff) < 0x3fc47ae1) {                // |h| < 0.16
+        const double x = h * h;
+        const float xf = d2f_scaled(x, 0);
+        sh = h * sinc_fp64(h, sct);
+        // cos h: terms from h^8 on in FP32 (rounding below 1e-18)
+        double p = f2d_bits(fmaf(xf, -1.0f / 3628800.0f, 1.0f / 40320.0f));
+        p = fma(x, p, -1.0 / 720.0);
+        p = fma(x, p, 1.0 / 24.0);
+        p = fma(x, p, -0.5);
+        ch = fma(x, p, 1.0);
+    } else {
+        sincos_tab(h, sct, sh, ch);
+    }
     double2 U[3], V[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -1846,6 +1859,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
             const int i0 = tid - pr * Tp2;
             typedef typename std::conditional<sizeof(R) == 8, double, float>::type Acc;
             Acc acc8[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // Crn (2), Cro (2), Hn, Ho, Cx (2)
+            const bool realsum = a.tdi2 != GBX_TDI2_BIT;
             // mixed form: FP32 sums over columns of the default tile's threads,
             // float pairs over the columns (as the likelihood)
             dfl tot8[8];
@@ -1885,6 +1899,25 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                             eR = d2f_scaled(dE.x, Bn.eD); eI = d2f_scaled(dE.y, Bn.eD);
                         }
                         const Acc hAr = hA.x, hAi = hA.y, hEr = hE.x, hEi = hE.y;
+                        if constexpr (sizeof(R) == 8) {
+                            if (realsum && K.A_psd == K.E_psd) {
+                                // one weight per bin; the imaginary parts only
+                                // meet complex (TDI-2) scales
+                                const Acc cr = fma(eI, hEi, fma(eR, hEr, fma(aI, hAi, aR * hAr)));
+                                const Acc hh2 = fma(hEi, hEi, fma(hEr, hEr, fma(hAi, hAi, hAr * hAr)));
+                                acc8[isnew ? 0 : 2] = fma(cr, wA, acc8[isnew ? 0 : 2]);
+                                acc8[isnew ? 4 : 5] = fma(hh2, wA, acc8[isnew ? 4 : 5]);
+                                const int k = j - Bo.start;
+                                if (isnew && k >= 0 && k < N) {
+                                    const int pk = bitrev((k + (N >> 1)) & (N - 1), lg);
+                                    const V oA = buf[(po * 2 + 0) * N + swz(pk, lg)],
+                                            oE = buf[(po * 2 + 1) * N + swz(pk, lg)];
+                                    acc8[6] = fma(fma(oE.y, hEi, fma(oE.x, hEr, fma(oA.y, hAi, oA.x * hAr))),
+                                                  wA, acc8[6]);
+                                }
+                                continue;
+                            }
+                        }
                         // conj(r) h / S
                         const Acc cr = (aR * hAr + aI * hAi) * wA + (eR * hEr + eI * hEi) * wE;
                         const Acc ci = (aR * hAi - aI * hAr) * wA + (eR * hEi - eI * hEr) * wE;
@@ -2054,9 +2087,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                             const double S = __ldg(K.A_psd + jn);
                             if constexpr (sizeof(R) == 8) {
                                 const double w = recip_fp64(S);
-                                sr = fma((dA.x * tA.x + dA.y * tA.y) + (dE.x * tE.x + dE.y * tE.y), w, sr);
-                                si = fma((dA.x * tA.y - dA.y * tA.x) + (dE.x * tE.y - dE.y * tE.x), w, si);
-                                sh = fma((tA.x * tA.x + tA.y * tA.y) + (tE.x * tE.x + tE.y * tE.y), w, sh);
+                                sr = fma(fma(dE.y, tE.y, fma(dE.x, tE.x, fma(dA.y, tA.y, dA.x * tA.x))), w, sr);
+                                si = fma(fma(-dE.y, tE.x, fma(dE.x, tE.y, fma(-dA.y, tA.x, dA.x * tA.y))), w, si);
+                                sh = fma(fma(tE.y, tE.y, fma(tE.x, tE.x, fma(tA.y, tA.y, tA.x * tA.x))), w, sh);
                             } else {
                                 const float w = __frcp_rn(d2f_scaled(S, B.eS));
                                 const float aR = d2f_scaled(dA.x, B.eD), aI = d2f_scaled(dA.y, B.eD);
