@@ -1289,6 +1289,39 @@ __device__ __forceinline__ void fft_dif(typename C2<R>::T *buf, int nsub, int lg
 // (+-1 - i)/sqrt2, and multiplies output k once by W^(r k): 84 instructions
 // per 8 elements instead of 96, 28 per 4 instead of 32.
 template <int RB>
+__device__ __forceinline__ void dft_small_d(double2 (&x)[1 << RB])
+{
+    constexpr int M = 1 << RB;
+#pragma unroll
+    for (int j = 0; j < RB; j++) {
+        const int dm = M >> (j + 1);
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            if (m & dm) continue;
+            const double2 u = x[m], t = csub(u, x[m + dm]);
+            x[m] = cadd(u, x[m + dm]);
+            // times exp(-i pi e / 4)
+            const int e = (m & (dm - 1)) * (4 / dm);
+            constexpr double h = 0.70710678118654752440;
+            if (e == 0) x[m + dm] = t;
+            else if (e == 2) x[m + dm] = make_double2(t.y, -t.x);
+            else if (e == 1) x[m + dm] = make_double2((t.x + t.y) * h, (t.y - t.x) * h);
+            else x[m + dm] = make_double2((t.y - t.x) * h, -(t.x + t.y) * h);
+        }
+    }
+}
+// register m of dft_small_d holds output k = bitrev(m); its factor W^(r k), the
+// table's half period continued by its sign
+template <int RB>
+__device__ __forceinline__ double2 twiddle_d(int r, int m, int ts)
+{
+    const int k = RB == 1 ? 1 : RB == 2 ? ((m & 1) << 1) | (m >> 1) : ((m & 1) << 2) | (m & 2) | (m >> 2);
+    const int idx = r * k * ts;
+    const double2 w = tw<double>(idx & (kTwN / 2 - 1));
+    return (idx & (kTwN / 2)) ? make_double2(-w.x, -w.y) : w;
+}
+
+template <int RB>
 __device__ __forceinline__ void fft_reg_pass_d(double2 *buf, int nsub, int lg, int hl)
 {
     constexpr int M = 1 << RB;
@@ -1305,35 +1338,10 @@ __device__ __forceinline__ void fft_reg_pass_d(double2 *buf, int nsub, int lg, i
         double2 x[M];
 #pragma unroll
         for (int m = 0; m < M; m++) x[m] = sub[swz(p0 + (m << q), lg)];
-#pragma unroll
-        for (int j = 0; j < RB; j++) {
-            const int dm = M >> (j + 1);
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                if (m & dm) continue;
-                const double2 u = x[m], t = csub(u, x[m + dm]);
-                x[m] = cadd(u, x[m + dm]);
-                // times exp(-i pi e / 4)
-                const int e = (m & (dm - 1)) * (4 / dm);
-                constexpr double h = 0.70710678118654752440;
-                if (e == 0) x[m + dm] = t;
-                else if (e == 2) x[m + dm] = make_double2(t.y, -t.x);
-                else if (e == 1) x[m + dm] = make_double2((t.x + t.y) * h, (t.y - t.x) * h);
-                else x[m + dm] = make_double2((t.y - t.x) * h, -(t.x + t.y) * h);
-            }
-        }
+        dft_small_d<RB>(x);
         sub[swz(p0, lg)] = x[0];
 #pragma unroll
-        for (int m = 1; m < M; m++) {
-            // register m holds output k = bitrev(m); W^(r k), the table's half
-            // period continued by its sign
-            const int k = RB == 1 ? 1 : RB == 2 ? ((m & 1) << 1) | (m >> 1)
-                                                : ((m & 1) << 2) | (m & 2) | (m >> 2);
-            const int idx = r * k * ts;
-            double2 w = tw<double>(idx & (kTwN / 2 - 1));
-            if (idx & (kTwN / 2)) w = make_double2(-w.x, -w.y);
-            sub[swz(p0 + (m << q), lg)] = cmul(x[m], w);
-        }
+        for (int m = 1; m < M; m++) sub[swz(p0 + (m << q), lg)] = cmul(x[m], twiddle_d<RB>(r, m, ts));
     }
 }
 
@@ -1543,6 +1551,195 @@ __device__ __forceinline__ void third_prepass(const Bin *bins, const double *__r
         }
     }
     __syncthreads();
+}
+
+// one bin's conj(d) h / S and |h|^2 / S added to the sums (gbgpu_utils.cu:172-178)
+__device__ __forceinline__ void ll_add_fp64(double2 dA, double2 dE, double2 tA, double2 tE, double SA, double SE,
+                                            bool same, double &sr, double &si, double &sh)
+{
+    const double wA = recip_fp64(SA);
+    if (same) {
+        // one PSD for both channels: their terms summed, then weighted once
+        sr = fma(fma(dE.y, tE.y, fma(dE.x, tE.x, fma(dA.y, tA.y, dA.x * tA.x))), wA, sr);
+        si = fma(fma(-dE.y, tE.x, fma(dE.x, tE.y, fma(-dA.y, tA.x, dA.x * tA.y))), wA, si);
+        sh = fma(fma(tE.y, tE.y, fma(tE.x, tE.x, fma(tA.y, tA.y, tA.x * tA.x))), wA, sh);
+        return;
+    }
+    const double wE = recip_fp64(SE);
+    sr += (dA.x * tA.x + dA.y * tA.y) * wA + (dE.x * tE.x + dE.y * tE.y) * wE;
+    si += (dA.x * tA.y - dA.y * tA.x) * wA + (dE.x * tE.y - dE.y * tE.x) * wE;
+    sh += (tA.x * tA.x + tA.y * tA.y) * wA + (tE.x * tE.x + tE.y * tE.y) * wE;
+}
+
+// one bin of the output windows, from the transformed channels
+__device__ __forceinline__ void wave_out_fp64(const KParams &K, const Bin &B, size_t o, int N, double2 X, double2 Y,
+                                              double2 Z)
+{
+    const double is2 = 0.70710678118654752440, is6 = 0.40824829046386301637;
+    const double2 Xd = cmul(X, B.scale), Yd = cmul(Y, B.scale), Zd = cmul(Z, B.scale);
+    if (K.XYZ) {
+        K.XYZ[o] = Xd;
+        K.XYZ[o + N] = Yd;
+        K.XYZ[o + 2 * N] = Zd;
+    }
+    if (K.AET) {
+        // utility.py:24-38, with the divisions by sqrt 2, 6, 3 as
+        // products with their reciprocals (<= 1 ulp apart)
+        const double i3 = 0.57735026918962576451;
+        K.AET[o] = make_double2((Zd.x - Xd.x) * is2, (Zd.y - Xd.y) * is2);
+        K.AET[o + N] = make_double2((Xd.x - 2.0 * Yd.x + Zd.x) * is6, (Xd.y - 2.0 * Yd.y + Zd.y) * is6);
+        K.AET[o + 2 * N] = make_double2((Xd.x + Yd.x + Zd.x) * i3, (Xd.y + Yd.y + Zd.y) * i3);
+    }
+}
+
+// ----------------------------------------------------------------------------
+// Few FP64 binaries: a cluster of 2^LC blocks, on as many SMs, per binary.
+// One block per binary keeps its SM's FP64 units busy and leaves the other SMs
+// idle.  Here block r builds the samples n = k N/2^LC + m of its N/4^LC values
+// of m (all k), so that the transform's first stages (one DFT over k) need no
+// exchange; their output k goes to the shared memory of block k, whose
+// remaining N/2^LC points are a transform of their own.  Then each block writes
+// its share of the window, or adds it to the sums, in runs of 32 bins read from
+// all blocks; block 0 adds up the sums.
+// MODE_WAVE and MODE_LL, equal arms, 9 parameters, one N, with a workspace.
+// Bound by the serial chain of one sample's FP64 instructions (a warp's cost 64
+// cycles each) and its set-up in prep_kernel, no longer by one SM's FP64 units.
+// One window of N = 1024: 133 -> 35 us, of N = 4096: 520 -> 80 us, both kernels.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// address in block `rank` of the cluster of what is at p in this block
+__device__ __forceinline__ unsigned cluster_addr(const void *p, int rank)
+{
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(unsigned a, double2 v)
+{
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ double2 cluster_load(unsigned a)
+{
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
+}
+
+template <int MODE, int LC>
+__global__ void __launch_bounds__(kBlock, 2) wave_cluster_kernel(const KParams K)
+{
+    constexpr int NCH = MODE == MODE_WAVE ? 3 : 2, ncl = 1 << LC;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const gbx_wave_args &a = K.a;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int slot = blockIdx.x >> LC, rank = blockIdx.x & (ncl - 1);
+    const int lg = 31 - __clz(a.N), N = 1 << lg, lq = lg - LC, lr = lq - LC, Q = 1 << lq;
+    Bin &B = *reinterpret_cast<Bin *>(smem);
+    double2 *red = reinterpret_cast<double2 *>(smem + sizeof(Bin));       // block 0: [ncl][2]
+    double2 *sct = red + 2 * ncl;
+    double2 *own = sct + kScN;              // [NCH][Q] this block's samples
+    double2 *buf = own + NCH * Q;           // [NCH][Q] this block's part of the transforms
+    __shared__ double part[kBlock / 32][3];
+    const double *tab = reinterpret_cast<const double *>(a.orbit[lg]);
+    for (int k = tid; k < kScN; k += kBlock) sct[k] = g_sc_d[k];
+    const int4 *src = reinterpret_cast<const int4 *>(static_cast<const Bin *>(a.workspace) + slot);
+    for (int k = tid; k < (int)(sizeof(Bin) / 16); k += kBlock) reinterpret_cast<int4 *>(smem)[k] = src[k];
+    __syncthreads();
+
+    const double step = a.T * exp2_int(-lg);
+    const bool chirp = fmaf(fabsf(B.fddotf), (float)a.T, fabsf(B.fdotf)) * K.T2f > 0.3f;
+    for (int q = tid; q < Q; q += kBlock) {
+        const int n = ((q >> lr) << lq) + (rank << lr) + (q & ((1 << lr) - 1));
+        double2 o[3];
+        if (B.valid) {
+            slow_fp64<false, NCH == 2>(B, n, N, f2d_bits((float)n) * step, tab, K.Loc, sct, chirp, nullptr, nullptr, o);
+        } else {
+            o[0] = o[1] = o[2] = make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int c = 0; c < NCH; c++) own[(c << lq) + q] = o[c];
+    }
+    // (every block of the cluster runs before any writes into its memory)
+    cluster_sync();
+    for (int g = tid; g < (NCH << lr); g += kBlock) {
+        const int c = g >> lr, ml = g & ((1 << lr) - 1), r = (rank << lr) + ml;
+        double2 x[ncl];
+#pragma unroll
+        for (int k = 0; k < ncl; k++) x[k] = own[(c << lq) + (k << lr) + ml];
+        dft_small_d<LC>(x);
+        const double2 *dst = buf + (c << lq) + swz(r, lq);
+        cluster_store(cluster_addr(dst, 0), x[0]);
+#pragma unroll
+        for (int m = 1; m < ncl; m++) cluster_store(cluster_addr(dst, m), cmul(x[m], twiddle_d<LC>(r, m, kTwN >> lg)));
+    }
+    cluster_sync();
+    fft_dif_d(buf, NCH, lq);
+    cluster_sync();
+
+    double sr = 0.0, si = 0.0, sh = 0.0;
+    bool out = false;
+    for (int i = (warp * ncl + rank) * 32 + lane; i < N; i += ncl * kBlock) {
+        const int pos = bitrev((i + (N >> 1)) & (N - 1), lg);    // fftshift
+        const unsigned h = cluster_addr(buf + swz(pos & (Q - 1), lq), pos >> lq);
+        if constexpr (MODE == MODE_WAVE) {
+            if (B.b < 0) continue;
+            wave_out_fp64(K, B, (size_t)B.b * 3 * N + i, N, cluster_load(h), cluster_load(h + (unsigned)(Q * 16)),
+                          cluster_load(h + (unsigned)(Q * 32)));
+            if (i == 0 && K.start_out) K.start_out[B.b] = B.start;
+        } else {
+            const int j = B.start + i;
+            if (!B.valid) continue;
+            if (j < 0 || j >= K.L) {
+                out = true;
+                continue;
+            }
+            const size_t jd = (size_t)B.di * K.L + j, jn = (size_t)B.ni * K.L + j;
+            const bool same = K.A_psd == K.E_psd;
+            const double SA = __ldg(K.A_psd + jn), SE = same ? SA : __ldg(K.E_psd + jn);
+            ll_add_fp64(__ldg(K.A_data + jd), __ldg(K.E_data + jd), cluster_load(h),
+                        cluster_load(h + (unsigned)(Q * 16)), SA, SE, same, sr, si, sh);
+        }
+    }
+    if constexpr (MODE == MODE_LL) {
+        if (out) flag(a.status, GBX_FLAG_WINDOW);
+        for (int o = 16; o > 0; o >>= 1) {
+            sr += __shfl_xor_sync(0xffffffffu, sr, o);
+            si += __shfl_xor_sync(0xffffffffu, si, o);
+            sh += __shfl_xor_sync(0xffffffffu, sh, o);
+        }
+        if (lane == 0) {
+            part[warp][0] = sr;
+            part[warp][1] = si;
+            part[warp][2] = sh;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double t[3] = {0.0, 0.0, 0.0};
+            for (int w = 0; w < kBlock / 32; w++)
+                for (int k = 0; k < 3; k++) t[k] += part[w][k];
+            cluster_store(cluster_addr(red + 2 * rank, 0), make_double2(t[0], t[1]));
+            cluster_store(cluster_addr(red + 2 * rank + 1, 0), make_double2(t[2], 0.0));
+        }
+    }
+    // (no block leaves while others read its memory)
+    cluster_sync();
+    if constexpr (MODE == MODE_LL) {
+        if (rank == 0 && tid == 0 && B.b >= 0) {
+            double2 d = make_double2(0.0, 0.0);
+            double h = 0.0;
+            for (int r = 0; r < ncl; r++) {
+                d = cadd(d, red[2 * r]);
+                h += red[2 * r + 1].x;
+            }
+            const double s4 = 4.0 * K.df;
+            const double ch = s4 * (B.scale.x * B.scale.x + B.scale.y * B.scale.y);
+            K.d_h[B.b] = B.valid ? cmul(make_double2(s4 * d.x, s4 * d.y), B.scale) : make_double2(0.0, 0.0);
+            K.h_h[B.b] = make_double2(B.valid ? ch * h : 0.0, 0.0);
+        }
+    }
 }
 
 // Third-body pre-passes of the mixed form for a tile of cnt binaries with
@@ -1810,22 +2007,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                   Z = buf[(p * 3 + 2) * N + swz(pos, lg)];
                 const size_t o = (size_t)B.b * 3 * N + i;
                 if constexpr (sizeof(R) == 8) {
-                    double2 Xd = cmul(X, B.scale), Yd = cmul(Y, B.scale), Zd = cmul(Z, B.scale);
-                    if (K.XYZ) {
-                        K.XYZ[o] = Xd;
-                        K.XYZ[o + N] = Yd;
-                        K.XYZ[o + 2 * N] = Zd;
-                    }
-                    if (K.AET) {
-                        // utility.py:24-38, with the divisions by sqrt 2, 6, 3 as
-                        // products with their reciprocals (<= 1 ulp apart)
-                        const double i3 = 0.57735026918962576451;
-                        K.AET[o] = make_double2((Zd.x - Xd.x) * is2, (Zd.y - Xd.y) * is2);
-                        K.AET[o + N] = make_double2((Xd.x - 2.0 * Yd.x + Zd.x) * is6,
-                                                    (Xd.y - 2.0 * Yd.y + Zd.y) * is6);
-                        K.AET[o + 2 * N] = make_double2((Xd.x + Yd.x + Zd.x) * i3,
-                                                        (Xd.y + Yd.y + Zd.y) * i3);
-                    }
+                    wave_out_fp64(K, B, o, N, X, Y, Z);
                 } else {
                     // mixed form: the channels and the scale in FP32 (the values
                     // carry FP32 accuracy), widened to FP64 on the integer pipe
@@ -2086,10 +2268,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                         if (samepsd) {
                             const double S = __ldg(K.A_psd + jn);
                             if constexpr (sizeof(R) == 8) {
-                                const double w = recip_fp64(S);
-                                sr = fma(fma(dE.y, tE.y, fma(dE.x, tE.x, fma(dA.y, tA.y, dA.x * tA.x))), w, sr);
-                                si = fma(fma(-dE.y, tE.x, fma(dE.x, tE.y, fma(-dA.y, tA.x, dA.x * tA.y))), w, si);
-                                sh = fma(fma(tE.y, tE.y, fma(tE.x, tE.x, fma(tA.y, tA.y, tA.x * tA.x))), w, sh);
+                                ll_add_fp64(dA, dE, tA, tE, S, S, true, sr, si, sh);
                             } else {
                                 const float w = __frcp_rn(d2f_scaled(S, B.eS));
                                 const float aR = d2f_scaled(dA.x, B.eD), aI = d2f_scaled(dA.y, B.eD);
@@ -2102,11 +2281,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                         }
                         const double SA = __ldg(K.A_psd + jn), SE = __ldg(K.E_psd + jn);
                         if constexpr (sizeof(R) == 8) {
-                            const double wA = recip_fp64(SA), wE = recip_fp64(SE);
-                            // conj(d) h / S  (gbgpu_utils.cu:172-178)
-                            sr += (dA.x * tA.x + dA.y * tA.y) * wA + (dE.x * tE.x + dE.y * tE.y) * wE;
-                            si += (dA.x * tA.y - dA.y * tA.x) * wA + (dE.x * tE.y - dE.y * tE.x) * wE;
-                            sh += (tA.x * tA.x + tA.y * tA.y) * wA + (tE.x * tE.x + tE.y * tE.y) * wE;
+                            ll_add_fp64(dA, dE, tA, tE, SA, SE, false, sr, si, sh);
                         } else {
                             const float2 hA = tA, hE = tE;
                             const float wA = __frcp_rn(d2f_scaled(SA, B.eS));
@@ -2283,6 +2458,20 @@ static size_t pair_smem_bytes(int maxS, int nch, int maxP)
            sizeof(float4) * (size_t)kScN + (size_t)nch * maxS * sizeof(cpx);
 }
 
+// per-binary constants into the workspace
+template <int MODE>
+static int launch_prep(const KParams &K, cudaStream_t st)
+{
+    const size_t psm = sizeof(Bin) * kPrepBlock;
+    auto pk = prep_kernel<MODE>;
+    int unused = 0;
+    const int rc = kernel_fit((const void *)pk, kPrepBlock, psm, &unused);
+    if (rc) return rc;
+    pk<<<(K.a.num_bin + kPrepBlock - 1) / kPrepBlock, kPrepBlock, psm, st>>>(K);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? GBX_OK : cuda_error(e, "prep_kernel launch");
+}
+
 // persistent launch of one tile kernel (after the per-binary prep_kernel when
 // the caller gave a workspace)
 template <int MODE>
@@ -2304,19 +2493,39 @@ static int launch_tiles(void (*kern)(const KParams), size_t sm, const KParams &K
         if (e != cudaSuccess) return cuda_error(e, "queue reset");
     }
     if (K.a.workspace) {
-        const size_t psm = sizeof(Bin) * kPrepBlock;
-        auto pk = prep_kernel<MODE>;
-        int unused = 0;
-        rc = kernel_fit((const void *)pk, kPrepBlock, psm, &unused);
+        rc = launch_prep<MODE>(K, st);
         if (rc) return rc;
-        pk<<<(K.a.num_bin + kPrepBlock - 1) / kPrepBlock, kPrepBlock, psm, st>>>(K);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_error(e, "prep_kernel launch");
     }
     kern<<<grid, kBlock, sm, st>>>(K);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "wave_kernel launch");
     return GBX_OK;
+}
+
+template <int MODE, int LC>
+static int launch_cluster(const KParams &K, cudaStream_t st)
+{
+    if (K.a.num_bin < 1) return GBX_OK;
+    auto kern = wave_cluster_kernel<MODE, LC>;
+    const size_t sm = sizeof(Bin) + sizeof(double2) * ((2 << LC) + kScN + (MODE == MODE_WAVE ? 6 : 4) * (size_t)(K.a.N >> LC));
+    int unused = 0;
+    int rc = kernel_fit((const void *)kern, kBlock, sm, &unused);
+    if (rc) return rc;
+    rc = launch_prep<MODE>(K, st);
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)K.a.num_bin << LC);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1u << LC;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, K);
+    return e == cudaSuccess ? GBX_OK : cuda_error(e, "wave_cluster_kernel launch");
 }
 
 template <typename R, int MODE, bool THIRD, bool UNEQ = false>
@@ -2356,6 +2565,19 @@ static int dispatch(KParams &K, int maxS, cudaStream_t st)
         }
     }
     if (K.a.precision == GBX_FP64) {
+        if constexpr (MODE == MODE_WAVE || MODE == MODE_LL) {
+            // Few binaries leave SMs idle under one block each: spread each over
+            // a cluster.  Windows of N = 1024 (512, 4096), us, clusters of 8, of
+            // 4, one block each: 1 binary 35 46 133 (32 32 72, 80 144 520); 30
+            // binaries 49 48 138 (35 33 75, 155 146 524); 57 binaries 85 77 138
+            // (57 47 76, 275 272 526); 76 binaries 116 106 137 (77 63 75, 340
+            // 397 525).  N = 256 at 57 binaries: 52 32 44, at 76: 69 49 44.  A
+            // cluster needs a run of 32 samples per block: N >= 256.
+            if (!third && !uneq && K.a.tiles == nullptr && K.a.workspace && K.a.blocks_per_sm == 0 && K.a.N >= 256) {
+                if (K.a.num_bin <= num_sms() / 8) return launch_cluster<MODE, 3>(K, st);
+                if (K.a.num_bin <= 3 * num_sms() / 8) return launch_cluster<MODE, 2>(K, st);
+            }
+        }
         if (uneq) return launch_one<double, MODE, false, true>(K, maxS, st);
         return third ? launch_one<double, MODE, true>(K, maxS, st)
                      : launch_one<double, MODE, false>(K, maxS, st);
