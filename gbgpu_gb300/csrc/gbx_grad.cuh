@@ -603,13 +603,28 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
         // (The third body's second pass goes on with the first one's FP32 sums,
         // so a thread has one column there and the caller keeps the default tile.)
         const int Tv = THIRD ? Tpb : (SWAP ? 2 : 1) * (kBlock / tile_pack(0, lg, SWAP ? 2 : 1));
+        // Between the passes and across a pass's columns no total stays in
+        // registers (38 of them spilled in the second pass): the first pass's
+        // sums are reduced before the second, and a column of the second leaves
+        // its sums in the shared memory of its own samples, which nobody reads
+        // again.  8,191 x 512 at 2048 samples per tile: 555 -> 521 us, 505 with
+        // one column per thread.
+        float2 *red2 = reinterpret_cast<float2 *>(red);
+        const bool leader = (tid & (width - 1)) == 0;
+        const int grp = tid / width;
+        auto reduce = [&](int k, dfl x) {
+            for (int o = width >> 1; o > 0; o >>= 1) {
+                dfl y = {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
+                x = df_add(x, y);
+            }
+            if (leader) red2[kGradAcc * grp + k] = make_float2(x.h, x.l);
+        };
         float acc[kGradAcc];
-        dfl tot[kGradAcc];
+        dfl tot[5];
 #pragma unroll
-        for (int k = 0; k < kGradAcc; k++) {
-            acc[k] = 0.0f;
-            tot[k] = dfl{0.f, 0.f};
-        }
+        for (int k = 0; k < kGradAcc; k++) acc[k] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 5; k++) tot[k] = dfl{0.f, 0.f};
         if (p < cnt) {
             const Bin &B = bins[p];
             bool out = false;
@@ -670,19 +685,24 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
                 buf[(p * 2 + 0) * N + sp] = make_float2(uA.x, -uA.y);
                 buf[(p * 2 + 1) * N + sp] = make_float2(uE.x, -uE.y);
             }
-            if (!THIRD) {
 #pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    tot[k] = df_add(tot[k], dfl{acc[k], 0.f});
-                    acc[k] = 0.f;
-                }
+            for (int k = 0; k < 5; k++) {
+                tot[k] = df_add(tot[k], dfl{acc[k], 0.f});
+                acc[k] = 0.f;
             }
           }
             if (out) flag(a.status, GBX_FLAG_WINDOW);
         }
+#pragma unroll
+        for (int k = 0; k < 5; k++) reduce(k, tot[k]);
         __syncthreads();
         fft_dit<float>(buf, 2 * cnt, lg);
 
+        auto column = [&](int f, int v) {
+            // (N / Tv >= 2 without SWAP; with it the current source's slots are free)
+            const int n0 = (p << lg) + v, n1 = SWAP ? n0 - N : n0 + Tv;
+            return f < 3 ? es + 3 * n0 + f : f < 6 ? es + 3 * n1 + (f - 3) : buf + p * 2 * N + swz(v, lg);
+        };
         // backward pass: Y_c,n at natural position n
         if (p < cnt) {
             const Bin &B = bins[p];
@@ -717,11 +737,12 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
                         slow_grad_mixed<false>(B, Gx, n, N, stepd, tab, ifs, fstarf, Yc, Es, acc + 5);
                     }
                 }
-                if (!THIRD) {
+                if constexpr (!THIRD) {
+                    static_assert(kGradAcc == 19, "seven float2 per column");
 #pragma unroll
-                    for (int k = 5; k < kGradAcc; k++) {
-                        tot[k] = df_add(tot[k], dfl{acc[k], 0.f});
-                        acc[k] = 0.f;
+                    for (int f = 0; f < 7; f++) {
+                        *column(f, v) = make_float2(acc[5 + 2 * f], acc[6 + 2 * f]);
+                        acc[5 + 2 * f] = acc[6 + 2 * f] = 0.f;
                     }
                 }
               }
@@ -769,19 +790,22 @@ __global__ void __launch_bounds__(kBlock, 2) grad_kernel(const GradParams GP)
         // (binary, output) forms the result.  Spreading the FP64 work over
         // lanes keeps it off the critical path (the FP64 pipe issues a warp
         // instruction per 64 cycles per SM sub-partition, whatever the mask).
-        float2 *red2 = reinterpret_cast<float2 *>(red);
         double *tsum = red + kGradAcc * kMaxPack;
-        {
-            const bool leader = (tid & (width - 1)) == 0;
-            const int g = tid / width;
+        if constexpr (THIRD) {
 #pragma unroll
-            for (int k = 0; k < kGradAcc; k++) {
-                dfl x = THIRD ? dfl{acc[k], 0.f} : tot[k];
-                for (int o = width >> 1; o > 0; o >>= 1) {
-                    dfl y = {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
-                    x = df_add(x, y);
-                }
-                if (leader) red2[kGradAcc * g + k] = make_float2(x.h, x.l);
+            for (int k = 5; k < kGradAcc; k++) reduce(k, dfl{acc[k], 0.f});
+        } else {
+#pragma unroll
+            for (int f = 0; f < 7; f++) {
+                dfl x = {0.f, 0.f}, y = {0.f, 0.f};
+                if (valid)
+                    for (int v = i0; v < Tv; v += Tpb) {
+                        const float2 c = *column(f, v);
+                        x = df_add(x, dfl{c.x, 0.f});
+                        y = df_add(y, dfl{c.y, 0.f});
+                    }
+                reduce(5 + 2 * f, x);
+                reduce(6 + 2 * f, y);
             }
         }
         __syncthreads();
