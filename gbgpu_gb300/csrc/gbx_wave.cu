@@ -416,10 +416,10 @@ __device__ float vlos_grad_mixed(dfl t, const Bin &B, float cosvarpi, float P2yr
 // FP64 arithmetic of the set-up and the FP64 form.  One FP64 warp instruction
 // occupies its scheduler's FP64 unit for 64 cycles (measured), against one
 // cycle for an FP32 one, so the form is bound by the number of FP64
-// instructions and everything below is arranged to need few of them: 381 per
-// sample for the whole likelihood, where every link with its own sincos and
-// the library's sin, sincos and divisions took 754 (10,001 binaries of uneven
-// N: 7.78 -> 4.07 ms; 2,003 windows of N = 512: 1.53 -> 0.84 ms).
+// instructions and everything below is arranged to need few of them: 343 per
+// sample for the whole likelihood at N = 128, where every link with its own
+// sincos and the library's sin, sincos and divisions took 754 (10,001 binaries
+// of uneven N: 7.78 -> 3.92 ms; 2,003 windows of N = 512: 1.53 -> 0.83 ms).
 // ----------------------------------------------------------------------------
 // sin x and cos x: table of cos, sin at j pi/128 (tab[j & 255]) and the Taylor
 // series on the remainder |r| <= pi/256 (next terms below 1e-17 and 2e-20),
@@ -1432,7 +1432,7 @@ __device__ __noinline__ double kepler_newton(double u, double l, double e, const
 // from those at u0.  x0l is what the rounding of x0 left off; it and the rounding
 // of n2 (x0 - T2) go into l.  A swap step of 1,024 pairs of N = 512 (1,971 FP64
 // instructions per sample with a starter, a Newton step, two sincos, sin and
-// atan2 per spacecraft, now 580): 3.64 -> 1.41 ms.
+// atan2 per spacecraft, now 558): 3.64 -> 1.36 ms.
 __device__ __forceinline__ void vlos3_fp64(const Bin &B, double x0, double x0l, double del1, double del2,
                                            const double2 *__restrict__ sct, double v[3])
 {

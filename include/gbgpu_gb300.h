@@ -110,7 +110,7 @@ int gbx_get_ll_ex(void *d_h, void *h_h, const void *A_template, const void *E_te
  * (gbgpu/cutils/gbgpu_utils.cu:167-179; the division by S as a product with
  * 1/S), for callers that want the FP64 result itself rather than one within
  * 1e-12 of sum |terms|.  Same arguments, edge rules and flags; 3x the time
- * of gbx_get_ll_ex on GB300 (0.63 against 0.21 ms for 50k windows of 256
+ * of gbx_get_ll_ex on GB300 (0.63 against 0.19 ms for 50k windows of 256
  * bins), whose FP64 rate is 1/64 of its FP32 rate.
  */
 int gbx_get_ll_fp64(void *d_h, void *h_h, const void *A_template, const void *E_template,
