@@ -88,29 +88,27 @@ int kernel_fit(const void *kern, int block, size_t smem, int *per_sm)
     if (e != cudaSuccess) return cuda_error(e, "cudaGetDevice");
     if (smem > 227 * 1024) return set_error(GBX_ERR_UNSUPPORTED, "tile needs %zu B of shared memory", smem);
     std::lock_guard<std::mutex> g(lock);
-    size_t limit = 0;
     for (int k = 0; k < used; k++) {
         const Entry &t = table[k];
-        if (t.kern != kern || t.dev != dev) continue;
-        if (t.smem == smem && t.block == block) {
-            *per_sm = t.per_sm;
-            return GBX_OK;
-        }
-        limit = t.smem > limit ? t.smem : limit;
+        if (t.kern != kern || t.dev != dev || t.smem != smem || t.block != block) continue;
+        *per_sm = t.per_sm;
+        return GBX_OK;
     }
-    if (smem > limit || limit == 0) {
+    // only ever raised: another thread may be about to launch with more
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, kern);
+    if (e != cudaSuccess) return cuda_error(e, "cudaFuncGetAttributes");
+    if ((int)smem > fa.maxDynamicSharedSizeBytes) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute");
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(carveout)");
     }
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(carveout)");
     int n = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem);
     if (e != cudaSuccess) return cuda_error(e, "occupancy");
     *per_sm = n;
-    // full: the oldest entry goes; its kernel's limit stands at least as high
-    // as the entries left say, which at worst sets it again
+    // full: the oldest entry goes (its kernel's limit stays)
     table[next] = Entry{kern, smem, dev, block, n};
     next = (next + 1) % kEntries;
     used = used < kEntries ? used + 1 : used;
