@@ -1599,9 +1599,10 @@ __device__ __forceinline__ void wave_out_fp64(const KParams &K, const Bin &B, si
 // of m (all k), so that the transform's first stages (one DFT over k) need no
 // exchange; their output k goes to the shared memory of block k, whose
 // remaining N/2^LC points are a transform of their own.  Then each block writes
-// its share of the window, or adds it to the sums, in runs of 32 bins read from
+// its share of the window, or adds it to the sums or the template, in runs of 32 bins read from
 // all blocks; block 0 adds up the sums.
-// MODE_WAVE and MODE_LL, equal arms, 9 parameters, one N, with a workspace.
+// MODE_WAVE, MODE_LL and MODE_FILL, equal arms, 9 parameters, one N, with a
+// workspace.
 // Bound by the serial chain of one sample's FP64 instructions (a warp's cost 64
 // cycles each) and its set-up in prep_kernel, no longer by one SM's FP64 units.
 // One window of N = 1024: 133 -> 35 us, of N = 4096: 520 -> 80 us, both kernels.
@@ -1689,6 +1690,15 @@ __global__ void __launch_bounds__(kBlock, 2) wave_cluster_kernel(const KParams K
             wave_out_fp64(K, B, (size_t)B.b * 3 * N + i, N, cluster_load(h), cluster_load(h + (unsigned)(Q * 16)),
                           cluster_load(h + (unsigned)(Q * 32)));
             if (i == 0 && K.start_out) K.start_out[B.b] = B.start;
+        } else if constexpr (MODE == MODE_FILL) {
+            const int j = B.start + i;
+            if (!B.valid || j < 0 || j >= K.L) continue;
+            const double2 hA = cmul(cluster_load(h), B.scale), hE = cmul(cluster_load(h + (unsigned)(Q * 16)), B.scale);
+            const size_t o = (size_t)B.gi * K.gstride + j;
+            atomicAdd(&K.A_glob[o].x, hA.x);
+            atomicAdd(&K.A_glob[o].y, hA.y);
+            atomicAdd(&K.E_glob[o].x, hE.x);
+            atomicAdd(&K.E_glob[o].y, hE.y);
         } else {
             const int j = B.start + i;
             if (!B.valid) continue;
@@ -2565,13 +2575,14 @@ static int dispatch(KParams &K, int maxS, cudaStream_t st)
         }
     }
     if (K.a.precision == GBX_FP64) {
-        if constexpr (MODE == MODE_WAVE || MODE == MODE_LL) {
+        if constexpr (MODE == MODE_WAVE || MODE == MODE_LL || MODE == MODE_FILL) {
             // Few binaries leave SMs idle under one block each: spread each over
             // a cluster.  Windows of N = 1024 (512, 4096), us, clusters of 8, of
             // 4, one block each: 1 binary 35 46 133 (32 32 72, 80 144 520); 30
             // binaries 49 48 138 (35 33 75, 155 146 524); 57 binaries 85 77 138
             // (57 47 76, 275 272 526); 76 binaries 116 106 137 (77 63 75, 340
-            // 397 525).  N = 256 at 57 binaries: 52 32 44, at 76: 69 49 44.  A
+            // 397 525).  N = 256 at 57 binaries: 52 32 44, at 76: 69 49 44.  Fills of
+            // N = 1024, cluster and one block each: 1 binary 34 120, 57 69 122.  A
             // cluster needs a run of 32 samples per block: N >= 256.
             if (!third && !uneq && K.a.tiles == nullptr && K.a.workspace && K.a.blocks_per_sm == 0 && K.a.N >= 256) {
                 if (K.a.num_bin <= num_sms() / 8) return launch_cluster<MODE, 3>(K, st);

@@ -103,3 +103,29 @@ def test_captured():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out[0], gb.XYZf) and torch.equal(out[1], gb.AETf)
+
+
+@pytest.mark.parametrize("N", [256, 1024, 4096])
+def test_fills(N):
+    """Templates against sums of the large batch's windows; some windows leave
+    the templates at either end."""
+    from gbgpu_gb300 import GBGPU
+    rng = np.random.default_rng(N)
+    p, gb, G, L = binaries(), GBGPU(), 3, N + 20
+    start = int(F0 * T) - N // 2 + 30
+    gb.run_wave(*p, N=N, T=T, dt=10.0)
+    win, first = gb.AETf[:, :2].clone(), gb.start_inds.cpu().numpy() - start
+    assert first.min() < 0 and first.max() + N > L
+    prm = torch.as_tensor(p, device="cuda")
+    group = rng.integers(0, G, MANY).astype(np.int32)
+    for B in few():
+        want = torch.zeros((G, 2, L), dtype=torch.complex128, device="cuda")
+        size = 0.0
+        for b in range(MANY - B, MANY):
+            lo, hi = max(first[b], 0), min(first[b] + N, L)
+            want[group[b], :, lo:hi] += win[b, :, lo - first[b]:hi - first[b]]
+            size += win[b].abs().square().sum().sqrt().item()
+        got = torch.zeros_like(want)
+        gb.add_to_templates(prm[:, MANY - B:].contiguous(), torch.as_tensor(group[MANY - B:], device="cuda"),
+                            got, start_freq_ind=start, N=N, T=T, dt=10.0, precision="fp64")
+        assert (got - want).abs().square().sum().sqrt().item() < tolerance(N) * size
