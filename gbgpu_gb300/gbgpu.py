@@ -1076,7 +1076,10 @@ class GBGPUBase(abc.ABC):
         base, extra = [pT[i] for i in range(9)], [pT[i] for i in range(9, pT.shape[0])]
         add_args = self.prepare_additional_args(*extra) if extra else ()
         N = self._resolve_N(N, base[0], base[1], T, extra, oversample)
-        prm = self._params(base, add_args) if extra else pT[:9].contiguous()
+        # a copy of the caller's array (pT may be a view of it): the windows of
+        # these parameters are formed on first access, after the call
+        prm = self._params(base, add_args) if extra else \
+            pT[:9].clone(memory_format=torch.contiguous_format)
         B = prm.shape[1]
         self.num_bin, self.N, self.df = B, N, 1 / T
         total_groups, nchannels, data_length = templates.shape
