@@ -1406,11 +1406,18 @@ __device__ __forceinline__ void fft_dif_d(double2 *buf, int nsub, int lg)
 // ----------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------
-// One Newton iteration after another on Kepler's equation from u (FP64), for
-// the third-body pre-pass where its series does not apply (periods of days,
-// eccentricities close to 1); at most 20.
-__device__ __noinline__ double kepler_newton(double u, double l, double e, const double2 *__restrict__ sct)
+// The eccentric anomaly at mean anomaly l (up to a multiple of 2 pi) by Newton's
+// iteration from the FP32 solve at l itself, for the third-body pre-pass where
+// its series does not apply (periods of days, eccentricities close to 1).  Two
+// steps are enough up to e = 1 - 1e-6, at any l; from another spacecraft's anomaly
+// the iteration can leave the root near periapsis (e = 0.99, anomalies 0.01 apart).
+__device__ __noinline__ double kepler_newton(double l, double e, float ef, const double2 *__restrict__ sct)
 {
+    constexpr double kRound = 6755399441055744.0;
+    const double k = fma(l, kInvTwoPi, kRound) - kRound;
+    l = fma(-k, kTwoPiLo, fma(-k, kTwoPi, l));
+    const float lf = d2f_scaled(l, 0), uf = kepler_solve_f(fminf(fabsf(lf), (float)kPi), ef);
+    double u = f2d_bits(lf < 0.0f ? -uf : uf);
     for (int it = 0; it < 20; it++) {
         double s, c;
         sincos_tab(u, sct, s, c);
@@ -1466,7 +1473,7 @@ __device__ __forceinline__ void vlos3_fp64(const Bin &B, double x0, double x0l, 
             const float xf = d2f_scaled(x, 0);
             i = fma(i1, x + f2d_bits(xf * fmaf(xf, xf, xf)), i1);
         } else {
-            const double u = kepler_newton(u0, s == 0 ? l : l - dm, e, sct);
+            const double u = kepler_newton(s == 0 ? l : l - dm, e, B.e2f, sct);
             sincos_tab(u, sct, sn, cs);
             i = 1.0 / fma(-eD, cs, 1.0);
         }
