@@ -223,7 +223,7 @@ __device__ __forceinline__ dfl sinc_pair(dfl a, const float4 *__restrict__ tab)
     return p_div(sn, a);
 }
 
-// sin(a)/a and cos(a) for a pair a >= 0: Taylor series in x = a^2 for
+// sin(a)/a and cos(a): Taylor series in x = a^2 for
 // x < 2.56 (terms to x^7; truncation below 5e-12 and 9e-11), the leading three
 // coefficients as pairs and the rest as an FP32 tail (at most 4e-10 of the
 // result); beyond that cos and sin from sincos_pair and one pair division.
@@ -393,7 +393,8 @@ __device__ __forceinline__ void slow_pair_links(const Bin &B, int n, int N, dfl 
     slow_pair_unequal<AE>(r, kr, fo, E, A, p_addf(base, dfl{B.w2 * tf * tf, 0.f}), tdi, sct, out);
 }
 
-// sum p and difference m of sin(a)/a at a = h + al and h - al (|al| <= h).
+// sum p and difference m of sin(a)/a at a = h + al and h - al (|al| <= |h|; h < 0
+// for a negative frequency).
 // With q+- = (h +- al)^2 = sig +- tau, sig = h^2 + al^2, tau = 2 h al, the
 // series' terms combine: with rho = sig^2 + tau^2
 //   p = 2 - sig/3 + rho/60 - sig (rho + 2 tau^2)/2520 + ...
@@ -406,7 +407,7 @@ __device__ __forceinline__ void slow_pair_links(const Bin &B, int n, int N, dfl 
 __device__ __forceinline__ void sinc_sum_pair(dfl h, dfl h2, dfl al, const float4 *__restrict__ tab,
                                               dfl &p, dfl &m)
 {
-    if (h.h + fabsf(al.h) < 1.6f) {
+    if (fabsf(h.h) + fabsf(al.h) < 1.6f) {
         const dfl sig = u_addf(h2, p_sqr(al));
         const dfl tau = p_mul(p_scale(h, 2.f), al);
         const dfl tau2 = p_sqr(tau), sig2 = p_sqr(sig);
@@ -541,7 +542,7 @@ __device__ __forceinline__ void slow_pair(const Bin &B, int n, int N, dfl step, 
     th[2] = u_add(Th, a01);
     // cos h, and sin h to relative accuracy (it scales the window through g4)
     dfl c, s;
-    if (h.h < 0.16f) {
+    if (fabsf(h.h) < 0.16f) {
         dfl S;
         sinc_cos_pair(h, sct, S, c);
         s = p_mul(h, S);
