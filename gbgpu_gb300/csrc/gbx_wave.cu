@@ -554,7 +554,8 @@ __device__ Trig setup_bin(Bin &B, const KParams &K, int b, int N, int mode)
     B.pi3fddot = (1.0 / 3.0 * kPi) * fddot;
     const bool lib = a.precision != GBX_PAIR;
     auto sc_of = [lib](double x, double &s, double &c) {
-        if (lib) {
+        // (the table's reduction is good up to |x| of 1e12)
+        if (lib || !(fabs(x) < 1e6)) {
             const double2 r = sincos_lib(x);
             s = r.x;
             c = r.y;

@@ -34,3 +34,12 @@ def worst(p, N, T):
 @pytest.mark.parametrize("sign", [1, -1])
 def test_carrier_of_either_sign(f0, sign):
     assert worst(binaries(64, 1, sign * f0), 128, 31557600.0) < 1e-9
+
+
+@pytest.mark.parametrize("row", [5, 6, 7, 8])           # iota, psi, lam, beta
+@pytest.mark.parametrize("size", [1e5, 1e7, 1e14, 1e17, 1e20, -1e16])
+def test_large_angles(row, size):
+    """Both forms reduce the same FP64 angle, however large."""
+    p = binaries(64, 2)
+    p[row] += size
+    assert worst(p, 128, 31557600.0) < 1e-10
