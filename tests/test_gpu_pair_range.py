@@ -43,3 +43,11 @@ def test_large_angles(row, size):
     p = binaries(64, 2)
     p[row] += size
     assert worst(p, 128, 31557600.0) < 1e-10
+
+
+@pytest.mark.parametrize("f0", [1e-3, 6e-3, 0.02])
+@pytest.mark.parametrize("fdot", [1e-15, 2e-14, 1e-12, 1e-11, -1e-11, 1e-10])
+def test_chirps(f0, fdot):
+    """A month of a strong chirp: the phase pi fdot T^2 is 2e3 rad at most, which
+    pairs hold to 2^-48 of it, 8e-12, so that 1e-10 holds as for slow sources."""
+    assert worst(binaries(64, 3, f0, fdot), 128, 2629800.0) < 1e-10
