@@ -1561,6 +1561,13 @@ __device__ __forceinline__ void third_prepass(const Bin *bins, const double *__r
     __syncthreads();
 }
 
+// the sum of conj(d) h / S times the output scale, which is real but for TDI-2: a
+// real product keeps an infinite sum (a bin of zero PSD) from meeting 0 * inf
+__device__ __forceinline__ double2 scaled_sum(double2 x, double2 scale)
+{
+    return scale.y == 0.0 ? make_double2(x.x * scale.x, x.y * scale.x) : cmul(x, scale);
+}
+
 // one bin's conj(d) h / S and |h|^2 / S added to the sums (gbgpu_utils.cu:172-178)
 __device__ __forceinline__ void ll_add_fp64(double2 dA, double2 dE, double2 tA, double2 tE, double SA, double SE,
                                             bool same, double &sr, double &si, double &sh)
@@ -1754,7 +1761,7 @@ __global__ void __launch_bounds__(kBlock, 2) wave_cluster_kernel(const KParams K
             }
             const double s4 = 4.0 * K.df;
             const double ch = s4 * (B.scale.x * B.scale.x + B.scale.y * B.scale.y);
-            K.d_h[B.b] = B.valid ? cmul(make_double2(s4 * d.x, s4 * d.y), B.scale) : make_double2(0.0, 0.0);
+            K.d_h[B.b] = B.valid ? scaled_sum(make_double2(s4 * d.x, s4 * d.y), B.scale) : make_double2(0.0, 0.0);
             K.h_h[B.b] = make_double2(B.valid ? ch * h : 0.0, 0.0);
         }
     }
@@ -2387,7 +2394,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
                 const double cd = sizeof(R) == 8 ? s4 : s4 * exp2_int(B.eS - B.eD);
                 const double ch = (sizeof(R) == 8 ? s4 : s4 * exp2_int(B.eS)) *
                                   (B.scale.x * B.scale.x + B.scale.y * B.scale.y);
-                dh = cmul(make_double2(cd * tr, cd * ti), B.scale);
+                dh = scaled_sum(make_double2(cd * tr, cd * ti), B.scale);
                 hv = make_double2(ch * th, 0.0);
                 if (!B.valid) {
                     dh = make_double2(0.0, 0.0);
