@@ -1,0 +1,32 @@
+// Which binaries a warp of a launch takes, and how many blocks that needs: plain
+// integer arithmetic, written apart from the kernels so that it can be checked on
+// the host at sizes no test can run.
+#pragma once
+
+#ifdef __CUDACC__
+#define GBX_HD __host__ __device__ __forceinline__
+#else
+#define GBX_HD inline
+#endif
+
+namespace gbx {
+
+// get_ll: a warp takes two binaries, a block of kLlBlock threads eight, and the
+// grid covers any int num_bin in one round.  Counted in warps, of which there are
+// at most 2^30, so that a binary and one more stride fit 32 unsigned bits; the
+// threads, 16 num_bin, would leave them from 2^28 binaries on.
+constexpr int kLlBlock = 128;
+
+GBX_HD unsigned ll_first_binary(unsigned block, unsigned thread)
+{
+    return 2 * (block * (kLlBlock / 32) + (thread >> 5));
+}
+
+GBX_HD unsigned ll_stride(unsigned blocks) { return 2 * blocks * (kLlBlock / 32); }
+
+GBX_HD unsigned ll_blocks(int num_bin)
+{
+    return (unsigned)(((long long)num_bin + 7) / 8);
+}
+
+}  // namespace gbx

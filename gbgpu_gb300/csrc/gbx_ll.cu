@@ -4,6 +4,7 @@
 // get_ll: one warp per two binaries (lanes interleaved by binary); fill: one
 // warp per binary, lanes along the window.
 #include "gbx_common.cuh"
+#include "gbx_index.h"
 #include "gbx_internal.h"
 
 namespace gbx {
@@ -31,8 +32,6 @@ __device__ __forceinline__ dfl pair_sum_df(dfl v)
     return v;
 }
 
-constexpr int kLlBlock = 128;
-
 // <d|h>, <h|h> per binary (gbgpu_utils.cu:124-210).  A warp takes two
 // binaries: lane 2q + t walks points q, q + 16, ... of binary b + t, so a
 // warp's template loads cover whole 32-byte sectors in the point-major layout
@@ -56,9 +55,9 @@ __global__ void __launch_bounds__(kLlBlock, 8) get_ll_kernel(
     int L, long long tsi, long long tsb, int num_data, int num_psd, int *status)
 {
     const int lane = threadIdx.x & 31, t = lane & 1, q = lane >> 1;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int b0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; b0 < num_bin; b0 += 2 * warps) {
-        const int b = b0 + t;
+    // (one round; the loop's code is 1 % faster than an if's)
+    for (unsigned b0 = ll_first_binary(blockIdx.x, threadIdx.x); b0 < (unsigned)num_bin; b0 += ll_stride(gridDim.x)) {
+        const int b = (int)b0 + t;
         const bool has = b < num_bin;                 // odd num_bin: the last warp's lane t = 1 idles
         const int s = has ? start_ind[b] : 0;
         const int drow = has && data_index ? data_index[b] : 0;
@@ -511,8 +510,7 @@ static int get_ll_launch(void *d_h, void *h_h, const void *A_template, const voi
     if (rc) return rc;
     // one warp per pair of binaries, in small blocks (a grid-stride loop over the
     // resident warps leaves the last of 2.6 rounds for 50,000 part empty)
-    const long long warps = ((long long)num_bin + 1) / 2, per = kLlBlock / 32;
-    get_ll_kernel<FP64><<<(unsigned)((warps + per - 1) / per), kLlBlock, 0, (cudaStream_t)stream>>>(
+    get_ll_kernel<FP64><<<ll_blocks(num_bin), kLlBlock, 0, (cudaStream_t)stream>>>(
         (double2 *)d_h, (double2 *)h_h, (const double2 *)A_template, (const double2 *)E_template,
         (const double2 *)A_data, (const double2 *)E_data, A_psd, E_psd, df, start_ind, M, num_bin,
         data_index, noise_index, data_length, t_stride_i, t_stride_b, num_data, num_psd, status);
