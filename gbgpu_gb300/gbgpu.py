@@ -225,7 +225,6 @@ class WavePlan:
             a.blocks_per_sm = self.blocks_per_sm
             self._fixed = a
         a = nat.WaveArgs.from_buffer_copy(self._fixed)
-        a._keep = (self, params, status)
         a.params = params.data_ptr()
         a.nparams, B = params.shape
         a.num_bin = B
@@ -241,6 +240,8 @@ class WavePlan:
                                        device=self.owner.device)
             a.workspace = self._ws.data_ptr()
             a.workspace_bytes = self._ws.numel() * 16
+        # the workspace by itself: a larger batch on this plan replaces it
+        a._keep = (self, params, status, self._ws)
         return a
 
 
