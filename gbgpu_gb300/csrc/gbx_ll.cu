@@ -3,6 +3,7 @@
 // templates, and the scatter-add of templates into global buffers.
 // get_ll: one warp per two binaries (lanes interleaved by binary); fill: one
 // warp per binary, lanes along the window.
+#include "gbx_bulk.h"
 #include "gbx_common.cuh"
 #include "gbx_index.h"
 #include "gbx_internal.h"
@@ -294,48 +295,26 @@ __global__ void __launch_bounds__(kBulkWarps * 32) fill_global_bulk_kernel(
         }
         return false;
     };
-    auto issue = [&](int k, const Item &it) {
+    auto load = [&](int k, const Item &it) {
         const unsigned bar = smem_addr(&bars[warp][k]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(it.bytes) : "memory");
         asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          smem_addr(buf + (size_t)k * kBulkBins)), "l"(it.src), "r"(it.bytes), "r"(bar) : "memory");
     };
-    Item items[kBulkStages];
-    int in = 0;                          // copies issued
-    bool more = true;
-    // one stage stays free for the reduction that still reads its chunk
-#pragma unroll
-    for (int k = 0; k < kBulkStages - 1; k++) {
-        if (more && (more = get(items[k]))) {
-            issue(k, items[k]);
-            in++;
-        }
-    }
-    bool ok = true;
-    for (int done = 0; done < in;) {
-#pragma unroll
-        for (int k = 0; k < kBulkStages; k++) {
-            if (done >= in) break;
-            const unsigned parity = (unsigned)(done / kBulkStages) & 1u;
-            unsigned ready = 0;
-            for (int poll = 0; poll < kBulkPolls && !ready; poll++)
-                asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                             "selp.u32 %0, 1, 0, p;\n}" : "=r"(ready) : "r"(smem_addr(&bars[warp][k])), "r"(parity) : "memory");
-            ok = ok && ready;
-            if (ready)
-                asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(
-                                 items[k].dst), "r"(smem_addr(buf + (size_t)k * kBulkBins)), "r"(items[k].bytes) : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            done++;
-            // the stage of the previous reduction: refill it once it has been read
-            const int kn = k == 0 ? kBulkStages - 1 : k - 1;
-            asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            if (more && (more = get(items[kn]))) {
-                issue(kn, items[kn]);
-                in++;
-            }
-        }
-    }
+    auto loaded = [&](int k, unsigned parity) -> bool {
+        unsigned ready = 0;
+        for (int poll = 0; poll < kBulkPolls && !ready; poll++)
+            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                         "selp.u32 %0, 1, 0, p;\n}" : "=r"(ready) : "r"(smem_addr(&bars[warp][k])), "r"(parity) : "memory");
+        return ready != 0;
+    };
+    auto add = [&](int k, const Item &it) {
+        asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(it.dst),
+                     "r"(smem_addr(buf + (size_t)k * kBulkBins)), "r"(it.bytes) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    };
+    auto read = [&]() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); };
+    const bool ok = bulk_pipeline<kBulkStages, Item>(get, load, loaded, add, read);
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (!ok) flag(status, GBX_FLAG_COPY);
 }

@@ -734,6 +734,8 @@ class GBGPUBase(abc.ABC):
                           "those bins were left out of the inner products")
         if st & nat.GBX_FLAG_TILE:
             raise RuntimeError("malformed tile schedule")
+        if st & nat.GBX_FLAG_COPY:
+            raise RuntimeError("a bulk copy did not complete")
 
     def get_ll(self, params, data, psd, phase_marginalize=False, start_freq_ind=0,
                data_index=None, noise_index=None, **kwargs):
