@@ -29,4 +29,15 @@ GBX_HD unsigned ll_blocks(int num_bin)
     return (unsigned)(((long long)num_bin + 7) / 8);
 }
 
+// Row-major fill: kBulkWarps warps a block, each takes binaries first, first +
+// stride, ...  64-bit: the step past the last binary of the largest batches leaves
+// 32 bits.
+constexpr int kBulkWarps = 2;
+
+GBX_HD long long bulk_first_binary(unsigned block, unsigned warp) { return (long long)block * kBulkWarps + warp; }
+
+GBX_HD long long bulk_stride(unsigned blocks) { return (long long)blocks * kBulkWarps; }
+
+GBX_HD int bulk_blocks(int num_bin) { return num_bin / kBulkWarps + (num_bin % kBulkWarps != 0); }
+
 }  // namespace gbx

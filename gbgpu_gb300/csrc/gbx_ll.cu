@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) fill_global_kernel(
 // four FP64 reductions per bin took 197 us waiting on their round trips (one
 // template, whose sums stay in L2: 168 -> 97 us).  64 to 512 bins a chunk, 3 to
 // 12 stages and 2 to 8 warps are within 5 %.
-constexpr int kBulkBins = 256, kBulkStages = 4, kBulkWarps = 2;
+constexpr int kBulkBins = 256, kBulkStages = 4;
 constexpr size_t kBulkSmem = (size_t)kBulkWarps * kBulkStages * kBulkBins * sizeof(double2);
 constexpr int kBulkPolls = 1 << 20;      // bounded waits: far beyond any copy
 
@@ -255,8 +255,9 @@ __global__ void __launch_bounds__(kBulkWarps * 32) fill_global_bulk_kernel(
     // Work items: chunk c of channel ch of binary b.  `get` walks this warp's
     // items in order and skips what lies outside the data (gbgpu_utils.cu:88-91).
     const int chunks = (M + kBulkBins - 1) / kBulkBins;
-    const int stride = gridDim.x * kBulkWarps;
-    int b = blockIdx.x * kBulkWarps + warp, c = 0, ch = 0;
+    const long long stride = bulk_stride(gridDim.x);
+    long long b = bulk_first_binary(blockIdx.x, warp);
+    int c = 0, ch = 0;
     struct Item {
         const double2 *src;
         double2 *dst;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32) fill_global_bulk_kernel(
             const long long lo = max((long long)i0, -(long long)s), hi = min((long long)i1, (long long)L - s);
             const bool have = goff >= 0 && hi > lo;
             if (have) {
-                it.src = (ch ? E_t : A_t) + (long long)b * tsb + lo;
+                it.src = (ch ? E_t : A_t) + b * tsb + lo;
                 it.dst = (ch ? E_g : A_g) + goff + s + lo;
                 it.bytes = (unsigned)(hi - lo) * (unsigned)sizeof(double2);
             }
@@ -555,7 +556,7 @@ extern "C" int gbx_fill_global_ex(void *A_glob, void *E_glob, const void *A_temp
         int per_sm = 0;
         rc = kernel_fit((const void *)fill_global_bulk_kernel, kBulkWarps * 32, kBulkSmem, &per_sm);
         if (rc) return rc;
-        const int need = (num_bin + kBulkWarps - 1) / kBulkWarps, cap = num_sms() * (per_sm > 0 ? per_sm : 1);
+        const int need = bulk_blocks(num_bin), cap = num_sms() * (per_sm > 0 ? per_sm : 1);
         fill_global_bulk_kernel<<<need < cap ? need : cap, kBulkWarps * 32, kBulkSmem, (cudaStream_t)stream>>>(
             (double2 *)A_glob, (double2 *)E_glob, (const double2 *)A_template,
             (const double2 *)E_template, start_ind, M, num_bin, group_index, data_length,

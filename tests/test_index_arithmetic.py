@@ -27,6 +27,11 @@ int main(int, char **v)
     printf("%u %u %u %u %u %u %u %u\n", blocks, ll_first_binary(0, 0), ll_first_binary(0, 32),
            ll_first_binary(0, end), ll_first_binary(blocks - 1, 0), ll_first_binary(blocks - 1, end),
            ll_first_binary(0, 0) + ll_stride(blocks), ll_first_binary(blocks - 1, end) + ll_stride(blocks));
+    // the row-major fill: its largest grid, and the walk of a warp of a smaller one
+    const unsigned grid = 1216, full = (unsigned)bulk_blocks(n);
+    long long walked = 0, b = bulk_first_binary(grid - 1, kBulkWarps - 1);
+    for (; b < n && walked < 10; walked++) b += bulk_stride(grid) * (n / 4096 + 1);
+    printf("%d %lld %lld %lld\n", bulk_blocks(n), bulk_first_binary(full - 1, 0), bulk_stride(full), b);
 }
 ''')
     exe = str(d / "p")
@@ -38,10 +43,18 @@ int main(int, char **v)
 @pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 2 ** 28 - 1, 2 ** 28, 2 ** 28 + 1, 2 ** 31 - 1])
 def test_ll_covers_every_binary_once(program, n):
     out = subprocess.run([program, str(n)], capture_output=True, text=True, check=True).stdout
-    blocks, first, second, end0, last_block, last, again, last_again = map(int, out.split())
+    blocks, first, second, end0, last_block, last, again, last_again = map(int, out.split()[:8])
     # warp w takes binaries 2w and 2w + 1, four warps a block
     assert (first, second, end0) == (0, 2, 6)
     assert blocks == -(-n // 8) and blocks < 2 ** 31
     assert last_block == 8 * (blocks - 1) < n
     assert last == 8 * (blocks - 1) + 6
     assert n <= again == 8 * blocks and last_again == again + last      # and stops after it
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 2 ** 28, 2 ** 31 - 2432, 2 ** 31 - 1])
+def test_row_major_fill_covers_every_binary(program, n):
+    out = subprocess.run([program, str(n)], capture_output=True, text=True, check=True).stdout
+    blocks, last_first, stride, end = map(int, out.split()[8:12])
+    assert blocks == -(-n // 2) and last_first == 2 * (blocks - 1) < n <= stride
+    assert end >= n                  # a warp's walk ends past the last binary, not below zero
