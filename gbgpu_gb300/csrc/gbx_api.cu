@@ -72,12 +72,26 @@ extern "C" int gbx_version(void) { return 100; }
 // device, block, shared memory), so they are set and asked for once each: three
 // driver calls less per launch (about 5 us of a small call).  A larger dynamic
 // shared memory limit serves smaller launches too, so it only grows.
-int kernel_fit(const void *kern, int block, size_t smem, int *per_sm)
+cudaLaunchConfig_t cluster_config(unsigned grid, int cluster, int block, size_t smem, cudaLaunchAttribute *attr)
+{
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+int kernel_fit(const void *kern, int block, size_t smem, int *fit, int cluster)
 {
     struct Entry {
         const void *kern;
         size_t smem;
-        int dev, block, per_sm;
+        int dev, block, cluster, fit;
     };
     constexpr int kEntries = 128;
     static std::mutex lock;
@@ -90,8 +104,8 @@ int kernel_fit(const void *kern, int block, size_t smem, int *per_sm)
     std::lock_guard<std::mutex> g(lock);
     for (int k = 0; k < used; k++) {
         const Entry &t = table[k];
-        if (t.kern != kern || t.dev != dev || t.smem != smem || t.block != block) continue;
-        *per_sm = t.per_sm;
+        if (t.kern != kern || t.dev != dev || t.smem != smem || t.block != block || t.cluster != cluster) continue;
+        *fit = t.fit;
         return GBX_OK;
     }
     // only ever raised: another thread may be about to launch with more
@@ -105,11 +119,20 @@ int kernel_fit(const void *kern, int block, size_t smem, int *per_sm)
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(carveout)");
     int n = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem);
-    if (e != cudaSuccess) return cuda_error(e, "occupancy");
-    *per_sm = n;
+    if (cluster == 1) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, block, smem);
+        if (e != cudaSuccess) return cuda_error(e, "occupancy");
+    } else {
+        cudaLaunchAttribute attr = {};
+        cudaLaunchConfig_t cfg = cluster_config(cluster, cluster, block, smem, &attr);
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();             // a size this device does not take: none fit
+            n = 0;
+        }
+    }
+    *fit = n;
     // full: the oldest entry goes (its kernel's limit stays)
-    table[next] = Entry{kern, smem, dev, block, n};
+    table[next] = Entry{kern, smem, dev, block, cluster, n};
     next = (next + 1) % kEntries;
     used = used < kEntries ? used + 1 : used;
     return GBX_OK;

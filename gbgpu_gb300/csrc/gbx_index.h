@@ -40,4 +40,16 @@ GBX_HD long long bulk_stride(unsigned blocks) { return (long long)blocks * kBulk
 
 GBX_HD int bulk_blocks(int num_bin) { return num_bin / kBulkWarps + (num_bin % kBulkWarps != 0); }
 
+// A few FP64 binaries: log2 of the blocks that work on each (0: tiles, one block or
+// less), by the number of binaries, the window and the SMs; `fits(lc)` says whether a
+// cluster of 2^lc blocks can be resident.  The measurements are at the dispatch.
+template <typename Fits>
+inline int cluster_log2(int num_bin, int N, int sms, Fits &&fits)
+{
+    if (N < 256) return 0;
+    if (num_bin <= sms / 8 && fits(3)) return 3;
+    if (num_bin <= 3 * sms / 8 && fits(2)) return 2;
+    return 0;
+}
+
 }  // namespace gbx

@@ -10,5 +10,10 @@ int ensure_init(cudaStream_t st);
 int gbx_twiddle_init(cudaStream_t st);
 
 // Prepares `kern` for launches of `block` threads with `smem` bytes of dynamic
-// shared memory on the current device and gives the resident blocks per SM.
-int kernel_fit(const void *kern, int block, size_t smem, int *per_sm);
+// shared memory on the current device and gives what fits: the resident blocks per
+// SM or, for clusters of `cluster` blocks, the resident clusters (0: it cannot be
+// launched so, as on a partition of a GPU).
+int kernel_fit(const void *kern, int block, size_t smem, int *fit, int cluster = 1);
+
+// A launch in clusters; `attr` has to live as long as the configuration is used.
+cudaLaunchConfig_t cluster_config(unsigned grid, int cluster, int block, size_t smem, cudaLaunchAttribute *attr);

@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "gbx_common.cuh"
+#include "gbx_index.h"
 #include "gbx_internal.h"
 
 extern "C" size_t gbx_wave_workspace_bytes(int num_bin);
@@ -2528,28 +2529,31 @@ static int launch_tiles(void (*kern)(const KParams), size_t sm, const KParams &K
 }
 
 template <int MODE, int LC>
+static size_t cluster_smem_bytes(int N)
+{
+    return sizeof(Bin) + sizeof(double2) * ((2 << LC) + kScN + (MODE == MODE_WAVE ? 6 : 4) * (size_t)(N >> LC));
+}
+
+// whether wave_cluster_kernel can be resident at all
+template <int MODE, int LC>
+static bool cluster_fits(const KParams &K)
+{
+    int n = 0;
+    const void *kern = (const void *)wave_cluster_kernel<MODE, LC>;
+    return kernel_fit(kern, kBlock, cluster_smem_bytes<MODE, LC>(K.a.N), &n, 1 << LC) == GBX_OK && n > 0;
+}
+
+template <int MODE, int LC>
 static int launch_cluster(const KParams &K, cudaStream_t st)
 {
     if (K.a.num_bin < 1) return GBX_OK;
-    auto kern = wave_cluster_kernel<MODE, LC>;
-    const size_t sm = sizeof(Bin) + sizeof(double2) * ((2 << LC) + kScN + (MODE == MODE_WAVE ? 6 : 4) * (size_t)(K.a.N >> LC));
-    int unused = 0;
-    int rc = kernel_fit((const void *)kern, kBlock, sm, &unused);
+    const int rc = launch_prep<MODE>(K, st);
     if (rc) return rc;
-    rc = launch_prep<MODE>(K, st);
-    if (rc) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)K.a.num_bin << LC);
-    cfg.blockDim = dim3(kBlock);
-    cfg.dynamicSmemBytes = sm;
-    cfg.stream = st;
     cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 1u << LC;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, K);
+    cudaLaunchConfig_t cfg = cluster_config((unsigned)K.a.num_bin << LC, 1 << LC, kBlock,
+                                            cluster_smem_bytes<MODE, LC>(K.a.N), &attr);
+    cfg.stream = st;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, wave_cluster_kernel<MODE, LC>, K);
     return e == cudaSuccess ? GBX_OK : cuda_error(e, "wave_cluster_kernel launch");
 }
 
@@ -2599,9 +2603,13 @@ static int dispatch(KParams &K, int maxS, cudaStream_t st)
             // 397 525).  N = 256 at 57 binaries: 52 32 44, at 76: 69 49 44.  Fills of
             // N = 1024, cluster and one block each: 1 binary 34 120, 57 69 122.  A
             // cluster needs a run of 32 samples per block: N >= 256.
-            if (!third && !uneq && K.a.tiles == nullptr && K.a.workspace && K.a.blocks_per_sm == 0 && K.a.N >= 256) {
-                if (K.a.num_bin <= num_sms() / 8) return launch_cluster<MODE, 3>(K, st);
-                if (K.a.num_bin <= 3 * num_sms() / 8) return launch_cluster<MODE, 2>(K, st);
+            // Where no cluster can be resident (a partition of a GPU), one block each.
+            if (!third && !uneq && K.a.tiles == nullptr && K.a.workspace && K.a.blocks_per_sm == 0) {
+                const int lc = cluster_log2(K.a.num_bin, K.a.N, num_sms(), [&](int l) {
+                    return l == 3 ? cluster_fits<MODE, 3>(K) : cluster_fits<MODE, 2>(K);
+                });
+                if (lc == 3) return launch_cluster<MODE, 3>(K, st);
+                if (lc == 2) return launch_cluster<MODE, 2>(K, st);
             }
         }
         if (uneq) return launch_one<double, MODE, false, true>(K, maxS, st);

@@ -31,7 +31,11 @@ int main(int, char **v)
     const unsigned grid = 1216, full = (unsigned)bulk_blocks(n);
     long long walked = 0, b = bulk_first_binary(grid - 1, kBulkWarps - 1);
     for (; b < n && walked < 10; walked++) b += bulk_stride(grid) * (n / 4096 + 1);
-    printf("%d %lld %lld %lld\n", bulk_blocks(n), bulk_first_binary(full - 1, 0), bulk_stride(full), b);
+    printf("%d %lld %lld %lld ", bulk_blocks(n), bulk_first_binary(full - 1, 0), bulk_stride(full), b);
+    // clusters where 8 and 4, only 4, only 8 and neither can be resident
+    for (int fit = 0; fit < 4; fit++)
+        printf("%d ", cluster_log2(n, v[2] ? atoi(v[2]) : 256, 152,
+                                   [&](int lc) { return lc == 3 ? fit == 0 || fit == 2 : fit < 2; }));
 }
 ''')
     exe = str(d / "p")
@@ -58,3 +62,10 @@ def test_row_major_fill_covers_every_binary(program, n):
     blocks, last_first, stride, end = map(int, out.split()[8:12])
     assert blocks == -(-n // 2) and last_first == 2 * (blocks - 1) < n <= stride
     assert end >= n                  # a warp's walk ends past the last binary, not below zero
+
+
+@pytest.mark.parametrize("n,N,want", [(1, 256, [3, 2, 3, 0]), (19, 4096, [3, 2, 3, 0]), (20, 512, [2, 2, 0, 0]),
+                                      (57, 256, [2, 2, 0, 0]), (58, 256, [0] * 4), (1, 128, [0] * 4)])
+def test_clusters_only_where_they_fit(program, n, N, want):
+    out = subprocess.run([program, str(n), str(N)], capture_output=True, text=True, check=True).stdout
+    assert list(map(int, out.split()[12:])) == want
