@@ -231,6 +231,13 @@ __global__ void __launch_bounds__(256) fill_global_kernel(
 // four FP64 reductions per bin took 197 us waiting on their round trips (one
 // template, whose sums stay in L2: 168 -> 97 us).  64 to 512 bins a chunk, 3 to
 // 12 stages and 2 to 8 warps are within 5 %.
+// A copy and a reduction cost about 0.3 ns whatever their length, so short windows
+// keep the warp per window.  Here and there (us), 400,000 windows into 1 and 8
+// templates: 32 bins 258, 278 and 173, 216; 40 bins 258, 285 and 212, 266; 48 bins
+// 260, 297 and 257, 312; 64 bins 264, 328 and 337, 404.  50,000 windows: 32 bins
+// 33, 34 and 31, 29; 48 bins 35, 44 and 39, 46; 64 bins 40, 49 and 50, 58; up to
+// 3,000 windows there is no difference.
+constexpr int kBulkMinBins = 48;
 constexpr int kBulkBins = 256, kBulkStages = 4;
 constexpr size_t kBulkSmem = (size_t)kBulkWarps * kBulkStages * kBulkBins * sizeof(double2);
 constexpr int kBulkPolls = 1 << 20;      // bounded waits: far beyond any copy
@@ -549,10 +556,9 @@ extern "C" int gbx_fill_global_ex(void *A_glob, void *E_glob, const void *A_temp
     if (group_stride < data_length) return set_error(GBX_ERR_ARG, "group_stride < data_length");
     int rc = ensure_init((cudaStream_t)stream);
     if (rc) return rc;
-    if (t_stride_i == 1 && M >= 8 &&
+    if (t_stride_i == 1 && M >= kBulkMinBins &&
         (((uintptr_t)A_glob | (uintptr_t)E_glob | (uintptr_t)A_template | (uintptr_t)E_template) & 15) == 0) {
-        // row-major templates: bulk copies and reductions (windows of a few bins
-        // are not worth a copy each)
+        // row-major templates: bulk copies and reductions
         int per_sm = 0;
         rc = kernel_fit((const void *)fill_global_bulk_kernel, kBulkWarps * 32, kBulkSmem, &per_sm);
         if (rc) return rc;
