@@ -607,19 +607,22 @@ class GBGPUBase(abc.ABC):
         """(tile, blocks_per_sm) for this workload: the autotuner's choice when
         autotuning is on (timing ``run`` on the first call), else the rule of
         ``default_tile``.  An unverified ``nkey`` (``trusted=False``) only looks
-        up a cached shape; a new one is filed under the contents' own key."""
-        if not self.autotune and np.ndim(N) == 0:
+        up a cached shape; a new one is filed under the contents' own key.  The
+        rule's shapes and the tuner's are kept apart: ``autotune`` may be
+        switched between calls."""
+        tuned = bool(self.autotune)
+        if not tuned and np.ndim(N) == 0:
             return self._tile(kind, precision, nparams, N, B), 0
         if nkey is None:
             nkey = int(N) if np.ndim(N) == 0 else _array_key(np.ascontiguousarray(N, dtype=np.int64))
-        ck = (kind, nkey, int(B), precision, bool(tdi2), int(nparams))
+        ck = (kind if tuned else kind + " rule", nkey, int(B), precision, bool(tdi2), int(nparams))
         shape = self._shapes.get(ck)
         if shape is None and not trusted and np.ndim(N) != 0:
             nkey = _array_key(np.ascontiguousarray(N, dtype=np.int64))
-            ck = (kind, nkey, int(B), precision, bool(tdi2), int(nparams))
+            ck = (kind if tuned else kind + " rule", nkey, int(B), precision, bool(tdi2), int(nparams))
             shape = self._shapes.get(ck)
         if shape is None:
-            if self.autotune:
+            if tuned:
                 from .autotune import default_tuner, workload_key
                 shape = default_tuner().tune(workload_key(kind, N, B, precision, tdi2, nparams), run)
             else:
