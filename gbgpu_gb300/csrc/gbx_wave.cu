@@ -451,9 +451,12 @@ __device__ __forceinline__ void sincos_tab(double x, const double2 *__restrict__
 
 // sin(a)/a from its Taylor series in a^2: 5 terms after the first for
 // |a| < 0.16, 7 for |a| < 0.5, 11 for |a| < 1.6 (next terms below 5e-20,
-// 4e-20, 5e-21), sincos_tab beyond.  The last 2, 3 and 5 of them are summed in
-// FP32 (at most 7e-20, 2e-18 and 3e-17 of rounding) and widened on the integer
-// pipe, and the ranges are told apart by the high word.
+// 4e-20, 5e-21), sincos_tab beyond.  The last 2, 3 and 4 of them are summed in
+// FP32 (at most 7e-20, 2e-18 and 3e-18 of rounding) and widened on the integer
+// pipe, and the ranges are told apart by the high word.  From |a| = 1.1 on the
+// rounding of a^2 and of the last two sums is kept (6 more instructions, for links
+// above 21 mHz only): relative error below 1.2e-16 up to 1.6, where sin(a) and a
+// division give 1.7e-16; without it 2.7e-16 at 1.6.
 __device__ __forceinline__ double sinc_fp64(double a, const double2 *__restrict__ tab)
 {
     const double x = a * a;
@@ -468,11 +471,18 @@ __device__ __forceinline__ double sinc_fp64(double a, const double2 *__restrict_
     } else if (hx < 0x40047ae1) {                           // x < 2.56
         float t = fmaf(xf, -1.0f / 25852016738884976640000.0f, 1.0f / 51090942171709440000.0f);
         t = fmaf(t, xf, -1.0f / 121645100408832000.0f);
-        t = fmaf(t, xf, 1.0f / 355687428096000.0f);
-        p = f2d_bits(fmaf(t, xf, -1.0f / 1307674368000.0f));
+        p = f2d_bits(fmaf(t, xf, 1.0f / 355687428096000.0f));
+        p = fma(x, p, -1.0 / 1307674368000.0);
         p = fma(x, p, 1.0 / 6227020800.0);
         p = fma(x, p, -1.0 / 39916800.0);
         p = fma(x, p, 1.0 / 362880.0);
+        if (hx >= 0x3ff35c29) {                             // x >= 1.21
+            p = fma(x, p, -1.0 / 5040.0);
+            p = fma(x, p, 1.0 / 120.0);
+            const double c = -1.0 / 6.0, q = fma(x, p, c), ql = fma(x, p, c - q) - 9.251858538542970e-18;
+            const double s = fma(x, q, 1.0);
+            return s + fma(x, ql, fma(fma(a, a, -x), q, fma(x, q, 1.0 - s)));
+        }
     } else {
         double s, c;
         sincos_tab(a, tab, s, c);
@@ -3036,6 +3046,10 @@ __global__ void math_selftest_kernel(const void *x, float *out, int n, int which
         out[i] = d2f_scaled(static_cast<const double *>(x)[i], e);
         return;
     }
+    if (which == 3) {
+        reinterpret_cast<double *>(out)[i] = sinc_fp64(static_cast<const double *>(x)[i], g_sc_d);
+        return;
+    }
     const float xi = static_cast<const float *>(x)[i];
     float a, b;
     if (which == 0) sincos_mod(xi, a, b);
@@ -3047,9 +3061,11 @@ __global__ void math_selftest_kernel(const void *x, float *out, int n, int which
 
 extern "C" int gbx_math_selftest(const void *x, float *out, int n, int which, int e, void *stream)
 {
-    if (n < 0 || (n > 0 && (!x || !out)) || which < 0 || which > 2)
+    if (n < 0 || (n > 0 && (!x || !out)) || which < 0 || which > 3)
         return set_error(GBX_ERR_ARG, "math selftest: bad arguments");
     if (n == 0) return GBX_OK;
+    const int rc = ensure_init((cudaStream_t)stream);
+    if (rc) return rc;
     gbx::math_selftest_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(x, out, n, which, e);
     const cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? GBX_OK : cuda_error(err, "math_selftest_kernel launch");
