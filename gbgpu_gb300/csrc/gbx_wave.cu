@@ -271,14 +271,15 @@ __device__ __forceinline__ float d2f_scaled(double x, int e)
 }
 
 // the same with ties to even and no scaling: (float)x for values in FP32's
-// normal range, zero below it
+// normal range, infinities and NaN, zero below it
 __device__ __forceinline__ float d2f_rn(double x)
 {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const int ne = (int)((hi >> 20) & 0x7ffu) - 896;
     unsigned mag = __funnelshift_l(lo, hi, 3) - (896u << 23) +
                    ((lo >> 28) & ((lo & 0x2fffffffu) != 0u ? 1u : 0u));
-    mag = ((unsigned)(ne - 1) < 254u) ? mag : (ne >= 255 ? 0x7f800000u : 0u);
+    const unsigned top = ne == 1151 && ((hi << 12) | lo) != 0u ? 0x7fffffffu : 0x7f800000u;   // NaN, infinity
+    mag = ((unsigned)(ne - 1) < 254u) ? mag : (ne >= 255 ? top : 0u);
     return __uint_as_float((hi & 0x80000000u) | (mag & 0x7fffffffu));
 }
 
@@ -3047,7 +3048,12 @@ __global__ void math_selftest_kernel(const void *x, float *out, int n, int which
         return;
     }
     if (which == 3) {
+        // (written as doubles)
         reinterpret_cast<double *>(out)[i] = sinc_fp64(static_cast<const double *>(x)[i], g_sc_d);
+        return;
+    }
+    if (which == 4) {
+        out[i] = d2f_rn(static_cast<const double *>(x)[i]);
         return;
     }
     const float xi = static_cast<const float *>(x)[i];
@@ -3061,7 +3067,7 @@ __global__ void math_selftest_kernel(const void *x, float *out, int n, int which
 
 extern "C" int gbx_math_selftest(const void *x, float *out, int n, int which, int e, void *stream)
 {
-    if (n < 0 || (n > 0 && (!x || !out)) || which < 0 || which > 3)
+    if (n < 0 || (n > 0 && (!x || !out)) || which < 0 || which > 4)
         return set_error(GBX_ERR_ARG, "math selftest: bad arguments");
     if (n == 0) return GBX_OK;
     const int rc = ensure_init((cudaStream_t)stream);

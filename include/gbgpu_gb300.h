@@ -371,7 +371,8 @@ int gbx_waveform_ll_noalloc(const gbx_wave_args *a, const gbx_ll_args *l, void *
  * omega L; which = 1: x is float, sin(a)/a and cos(a) of the link transfer
  * functions; which = 2: x is double, out[i] = x[i] * 2^e rounded to FP32 by
  * the integer-pipe conversion of the mixed likelihood; which = 3: x is double,
- * out holds n doubles, sin(x[i])/x[i] of the FP64 form's links.
+ * out holds n doubles, sin(x[i])/x[i] of the FP64 form's links; which = 4: x is
+ * double, out[i] = x[i] rounded to FP32 by the set-up's conversion.
  */
 int gbx_math_selftest(const void *x, float *out, int n, int which, int e, void *stream);
 
