@@ -121,6 +121,15 @@ def plan_tiles(N_per_bin, tile=0):
     return order, tiles
 
 
+def _counts(N):
+    """(N, binaries) of each N in an array."""
+    N = np.asarray(N).reshape(-1)
+    if N.size and N.min() >= 0 and N.max() <= 8192:
+        c = np.bincount(N)
+        return [(int(n), int(c[n])) for n in np.flatnonzero(c)]
+    return [(int(n), int(c)) for n, c in zip(*np.unique(N, return_counts=True))]
+
+
 def default_tile(kind, precision, nparams, counts, sms):
     """Samples per tile when the autotuner is off, from the sizes alone.
 
@@ -632,17 +641,16 @@ class GBGPUBase(abc.ABC):
             self._shapes[ck] = shape
         return shape
 
-    def _tile(self, kind, precision, nparams, N, B):
-        """``default_tile`` for N (or one N per binary) on this device."""
+    def _tile(self, kind, precision, nparams, N, B, nkey=None):
+        """``default_tile`` for N (or one N per binary, kept under its content
+        key ``nkey`` where the caller has it) on this device."""
         key = None
-        if np.ndim(N) == 0:
-            counts = ((int(N), int(B)),)
-            key = (kind, precision, nparams, counts)
+        if np.ndim(N) == 0 or nkey is not None:
+            key = (kind, precision, nparams, int(N) if nkey is None else nkey, int(B))
             tile = self._tiles.get(key)
             if tile is not None:
                 return tile
-        else:
-            counts = [(int(n), int(c)) for n, c in zip(*np.unique(N, return_counts=True))]
+        counts = [(int(N), int(B))] if np.ndim(N) == 0 else _counts(N)
         if self._sms is None:
             self._sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         tile = default_tile(kind, precision, int(nparams), counts, self._sms)
@@ -1115,8 +1123,9 @@ class GBGPUBase(abc.ABC):
         work[:, 0:2].zero_()
         self._status.zero_()
         if B:
+            nkey = None if np.ndim(N) == 0 else _array_key(N)
             plan = self._plan(N, T, precision, tdi2, prm.shape[0],
-                              self._fill_tile(N, sort, precision, prm))
+                              self._fill_tile(N, sort, precision, prm, nkey), nkey=nkey)
             a = plan.args(prm, start_freq_ind, self._status)
             if sort:
                 self._fill_order(a, prm, gi, T, N)
@@ -1176,12 +1185,12 @@ class GBGPUBase(abc.ABC):
             nat.stream_handle())
         nat.check(rc, "gbx_waveform_fill")
 
-    def _fill_tile(self, N, sort, precision, prm):
+    def _fill_tile(self, N, sort, precision, prm, nkey=None):
         """Samples per tile of a fill: sorted fills pack up to 16 binaries (at
         most 4096 samples) so that neighbours share a tile; else the rule of
         ``default_tile``."""
         if not sort or np.ndim(N) != 0:
-            return self._tile("fill", precision, prm.shape[0], N, prm.shape[1])
+            return self._tile("fill", precision, prm.shape[0], N, prm.shape[1], nkey)
         return int(min(16 * int(N), 4096))
 
     @staticmethod

@@ -31,3 +31,21 @@ def test_switching_the_autotuner(monkeypatch):
     assert shape() == (1024, 2) and shape() == (1024, 2) and tuner.calls == 1
     gb.autotune = False
     assert shape() == rule and tuner.calls == 1
+
+
+def test_tile_of_an_array_is_found_once(monkeypatch):
+    from gbgpu_gb300 import gbgpu as G
+    rng = np.random.default_rng(1)
+    N = 2 ** rng.integers(5, 14, 3000)
+    n, c = np.unique(N, return_counts=True)
+    want = list(zip(n.tolist(), c.tolist()))
+    assert G._counts(N) == want
+    assert G._counts(np.array([-64, 64, 64, 2 ** 40])) == [(-64, 1), (64, 2), (2 ** 40, 1)]
+    assert G._counts(np.zeros(0, np.int64)) == []
+    gb = object.__new__(GBGPU)
+    gb._tiles, gb._sms, calls = {}, 152, []
+    monkeypatch.setattr(G, "_counts", lambda x: calls.append(1) or want)
+    for _ in range(3):
+        assert gb._tile("fill", "pair", 9, N, N.size, nkey=(1, 2)) == \
+            G.default_tile("fill", "pair", 9, want, 152)
+    assert len(calls) == 1
