@@ -531,7 +531,17 @@ __device__ __forceinline__ void slow_pair(const Bin &B, int n, int N, dfl step, 
     }
     dfl hp = h;
     hp.l = fmaf(-0.5f, dl, hp.l);
-    const dfl h2 = p_sqr(hp);
+    dfl h2 = p_sqr(hp);
+    // Strong chirps: f/f* at spacecraft s is off that at spacecraft 1 by -Kf kk, so
+    // the sinc arguments are a+ = (h' - Kf kk/2) (1 + k.r), a- = (h' - Kf (kk + k.r)/2)
+    // (1 - k.r): half sum h' + dh, half difference al + da (da = -+dh where one of the
+    // two links is spacecraft 1's).  sin(a)/a moves by up to 15 fdot, 1e-13 where the
+    // line lies: a month of fdot = 1e-11 (1e-10) at 4-8 mHz, windows within 4.3e-12
+    // (9.4e-12) of the FP64 form, 1.5e-10 (1.5e-9) without.  200,000 binaries 10,299
+    // us without the test, 10,367 with it, 10,387 with the shift for all of them,
+    // 10,500 with a second instantiation of this function.
+    const bool chirp = fabsf(Kf) > 3e-12f;
+    float dhp = 0.f;                     // the shift that hp and h2 hold
     dfl al[3], th[3];
     al[0] = p_mul(kr[0], hp);
     al[1] = p_mul(kr[1], hp);
@@ -552,18 +562,17 @@ __device__ __forceinline__ void slow_pair(const Bin &B, int n, int N, dfl step, 
     cpx U[3], V[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        // f/f* at spacecraft s is off that at spacecraft 1 by -Kf kk, so the sinc
-        // arguments are a+ = (h' - Kf kk/2) (1 + k.r), a- = (h' - Kf (kk + k.r)/2) (1 - k.r):
-        // half sum h' + dh, half difference al + da (da = -+dh where one of the
-        // two links is spacecraft 1's), which matters for strong chirps only (sin(a)/a
-        // moves by up to 15 fdot).  A month of fdot = 1e-11 (1e-10) at 4-8 mHz:
-        // windows within 4.6e-12 (9e-12) of the FP64 form, 1.5e-10 (1.5e-9) without.
-        const float k = krf[a], k2 = k * k, kf4 = -0.25f * Kf;
-        const float dh = kf4 * (a == 0 ? k - k2 : a == 1 ? fmaf(2.f, krf[0], k - k2) : -k - k2);
-        const float da = a == 0 ? -dh : a == 2 ? dh : kf4 * fmaf(2.f * krf[0], k, k2 - k);
         dfl p, m;
-        sinc_sum_pair(dfl{hp.h, hp.l + dh}, dfl{h2.h, fmaf(hp.h + hp.h, dh, h2.l)}, dfl{al[a].h, al[a].l + da},
-                      sct, p, m);
+        if (chirp) {
+            const float k = krf[a], k2 = k * k, kf4 = -0.25f * Kf;
+            const float dh = kf4 * (a == 0 ? k - k2 : a == 1 ? fmaf(2.f, krf[0], k - k2) : -k - k2);
+            const float da = a == 0 ? -dh : a == 2 ? dh : kf4 * fmaf(2.f * krf[0], k, k2 - k);
+            hp.l += dh - dhp;
+            h2.l = fmaf(hp.h + hp.h, dh - dhp, h2.l);
+            al[a].l += da;
+            dhp = dh;
+        }
+        sinc_sum_pair(hp, h2, al[a], sct, p, m);
         // antenna pattern r.e.r of the rotated basis, with the 1/4 of the
         // transfer functions
         const cpx A = {p_mul(B.pr.ap4, u_dot2(rv[a], rv[a], df_neg(ru[a]), ru[a])),
