@@ -495,8 +495,9 @@ __device__ __forceinline__ double sinc_fp64(double a, const double2 *__restrict_
     return fma(x, p, 1.0);
 }
 
-// 1 / x: the hardware's ~20-bit estimate and two Newton steps (relative error
-// after them ~1 ulp); the division for zero, subnormal, huge and non-finite x.
+// 1 / x: the hardware's ~20-bit estimate and two Newton-Raphson steps, whose last
+// rounding is all that is left (equal to the division for each of 5e8 random x); the
+// division for zero, subnormal, huge and non-finite x.
 __device__ __forceinline__ double recip_fp64(double x)
 {
     const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
@@ -2272,7 +2273,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 3 : 2) wave_kernel(co
             // data/PSD window.  Sums are FP64 (plain form) or, in the mixed form,
             // FP32 over the bins v, v + Tv, v + 2 Tv ... of a column v, Tv being
             // the threads a binary has in a tile of kTileMin samples, and in
-            // float pairs over the columns: the FP32 sums (2 to 8 terms), and
+            // float pairs over the columns: the FP32 sums (2 to 32 terms), and
             // so the result, do not depend on the tile.  Lanes are combined with
             // an FP64 or float-pair shuffle tree, and a binary's <= 16 group
             // partials are added by one thread per (binary, term).
@@ -2613,7 +2614,9 @@ static int dispatch(KParams &K, int maxS, cudaStream_t st)
             // (57 47 76, 275 272 526); 76 binaries 116 106 137 (77 63 75, 340
             // 397 525).  N = 256 at 57 binaries: 52 32 44, at 76: 69 49 44.  Fills of
             // N = 1024, cluster and one block each: 1 binary 34 120, 57 69 122.  A
-            // cluster needs a run of 32 samples per block: N >= 256.
+            // cluster needs a run of 32 samples per block: N >= 256.  The upper line is
+            // where N = 256 crosses; longer windows would still gain at half as many
+            // binaries as SMs.
             // Where no cluster can be resident (a partition of a GPU), one block each.
             if (!third && !uneq && K.a.tiles == nullptr && K.a.workspace && K.a.blocks_per_sm == 0) {
                 const int lc = cluster_log2(K.a.num_bin, K.a.N, num_sms(), [&](int l) {

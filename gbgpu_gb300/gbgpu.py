@@ -138,7 +138,7 @@ def default_tile(kind, precision, nparams, counts, sms):
     (N, binaries).  Upper end: the largest tile whose buffers leave an SM as
     many blocks as the registers do (three for the mixed form's likelihood,
     fill, swap and waveform kernels, two otherwise; bytes per sample below).
-    On one GB300, against 512 samples (us): gradient 8,191 x 512 691 -> 506,
+    On one GB300, against 512 samples (us): gradient 8,191 x 512 691 -> 521,
     mixed likelihood 50,000 x 256 660 -> 518, pair 1,314 -> 1,134, pair fill
     60,000 x 512 3,466 -> 3,016; one step further costs 10-30 %.  The FP64 form
     is bound by its FP64 instructions at any tile and stays at 512 (3,000 x

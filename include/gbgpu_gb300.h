@@ -35,7 +35,8 @@ extern "C" {
 #define GBX_FLAG_COPY 8        /* a bulk copy did not complete in time: its bins are missing */
 
 /* ---- precision of the waveform family ---- */
-#define GBX_FP64 0             /* every step in FP64 (the plain form) */
+#define GBX_FP64 0             /* FP64 accuracy throughout (the plain form); small terms whose FP32
+                                  rounding lies below an FP64 one's are formed in FP32 */
 #define GBX_MIXED 1            /* FP64 carrier phase, delays and reductions; FP32 slow part + FFT */
 #define GBX_PAIR 2             /* slow part, FFT and <d|h> in float pairs (FP32 pipe, ~44 bits);
                                   waveform, likelihood, fill and swap entry points,
